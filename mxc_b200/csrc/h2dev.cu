@@ -2066,13 +2066,10 @@ class Solver : public SolverBase {
       poff[i + 1] = poff[i] + Mr;
     }
     lv.B.alloc(std::max<i64>(1, lv.boff[nodes]));
-    // Global LU scratch only for redundant blocks too large for the solve
-    // kernel's shared memory; released at the end of the level.
-    i64 maxMr = 0;
-    for (i64 i = 0; i < nodes; i++) maxMr = std::max(maxMr, D[i] - Rk[i]);
-    const bool lu_in_smem = (double)sizeof(T) * maxMr * (maxMr + 1) + 8. * maxMr + 16. <= 200. * 1024.;
-    lv.invT.alloc(lu_in_smem ? 1 : std::max<i64>(1, lv.ioff[nodes]));
-    lv.ipiv.alloc(std::max<i64>(1, poff[nodes]));
+    // The factors of the redundant blocks (released at the end of the level),
+    // their pivots and row orders.
+    lv.invT.alloc(std::max<i64>(1, lv.ioff[nodes]));
+    lv.ipiv.alloc(std::max<i64>(1, 2 * poff[nodes]));
     lv.info.alloc(nodes);
     lv.info.zero(st());
     T* A = lv.A.p;
@@ -2114,8 +2111,9 @@ class Solver : public SolverBase {
       t.m = M;
       t.X = V + lv.qoff[i] + (i64)Ms * M;
       t.ldx = M;
-      t.work = lu_in_smem ? nullptr : lv.invT.p + lv.ioff[i];
+      t.work = lv.invT.p + lv.ioff[i];
       t.ipiv = lv.ipiv.p + poff[i];
+      t.prow = lv.ipiv.p + poff[nodes] + poff[i];
       t.info = lv.info.p + i;
       lt.push_back(t);
     }
@@ -2127,9 +2125,12 @@ class Solver : public SolverBase {
       double fl = 0.;
       for (const auto& t : lt) fl += 2. / 3. * (double)t.n * t.n * t.n + 2. * (double)t.n * t.n * t.m;
       Prof pf("lu_solve", fl, 0.);
-      int maxn = 0;
-      for (const auto& x : lt) maxn = std::max(maxn, x.n);
-      ck(launch_lu_solve<T>(dl.p, (int)lt.size(), maxn, st()), "lu_solve");
+      int maxn = 0, maxm = 0;
+      for (const auto& x : lt) {
+        maxn = std::max(maxn, x.n);
+        maxm = std::max(maxm, x.m);
+      }
+      ck(launch_lu_solve<T>(dl.p, (int)lt.size(), maxn, maxm, st()), "lu_solve");
     }
     // Steps 6-8.
     for (i64 i = 0; i < nodes; i++) {

@@ -233,21 +233,11 @@ template <typename T>
 cudaError_t launch_set_identity(T* base, const i64* qoff, const i64* dims, int nboxes, cudaStream_t st);
 
 // ---------------------------------------------------------------- lu
-template <typename T>
-struct LuTask {
-  T* A;      // n x n column-major (read only)
-  i64 lda;
-  int n;
-  T* invT;   // receives A^{-1} transposed (column-major, ld = ldinv)
-  i64 ldinv;
-  int* ipiv;  // n
-  int* info;  // 1 when |det| <= DBL_MIN (h2matrix.cpp:384)
-};
-template <typename T>
-cudaError_t launch_lu_inverse(const LuTask<T>* d_tasks, int ntasks, int maxn, cudaStream_t st);
-// PartialPivLU of A (n x n) and X = A^{-1} B for m right-hand sides stored
-// row by row: B[c + r ldb], X[c + r ldx] (r < n, c < m).  work: n x n scratch
-// (ld n) used when the factor does not fit in shared memory.
+// PartialPivLU of A (n x n, read only) and X = A^{-1} B for m right-hand sides
+// stored row by row: B[c + r ldb], X[c + r ldx] (r < n, c < m).  work (n x n,
+// ld n) receives the factor, ipiv the pivots, prow the row of B that lands in
+// each row of P B (n entries each), info 1 when |det| <= DBL_MIN
+// (h2matrix.cpp:384).  maxn, maxm: the largest n and m of the tasks, n <= 2048.
 template <typename T>
 struct LuSolveTask {
   const T* A;
@@ -260,10 +250,11 @@ struct LuSolveTask {
   i64 ldx;
   T* work;
   int* ipiv;
+  int* prow;
   int* info;
 };
 template <typename T>
-cudaError_t launch_lu_solve(const LuSolveTask<T>* d_tasks, int ntasks, int maxn, cudaStream_t st);
+cudaError_t launch_lu_solve(const LuSolveTask<T>* d_tasks, int ntasks, int maxn, int maxm, cudaStream_t st);
 
 // ---------------------------------------------------------------- vectors
 template <typename Ts, typename Td>

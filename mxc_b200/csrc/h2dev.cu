@@ -1116,7 +1116,7 @@ class Solver : public SolverBase {
   }
 
   // h2matrix.cpp:72-249 for one level.
-  // Ranks of fixed-rank bases (epi >= 1), by the rule k_basis_finish
+  // Ranks of fixed-rank bases (epi >= 1), by the rule k_interp
   // applies on the device: min(K, M, floor(epi)) with K the box's sample
   // rows (0 when K or M is 0).  Knowing them on the host spares the level a
   // device-to-host synchronisation before its completion plans are built.
@@ -1395,7 +1395,7 @@ class Solver : public SolverBase {
           }
           Prof pf("cpqr", fl, 0.);
           ck(launch_cpqr<T>(lv.d_dims.p, d_krows.p, Rws.p, lv.d_qoff.p, d_perm.p, lv.d_xoff.p, d_maxpiv.p,
-                            d_nonzero.p, cap, (int)nodes, (int)lv.maxM, st()),
+                            d_nonzero.p, cap, e, (int)nodes, (int)lv.maxM, st()),
              "cpqr");
         }
         DVec<T> taus;
@@ -1404,7 +1404,7 @@ class Solver : public SolverBase {
           Prof pfin("basis_finish", 0., (double)lv.qoff[nodes] * sizeof(T) * 3.);
           ck(launch_basis_finish<T>(lv.d_dims.p, d_krows.p, Rws.p, lv.Q.p, lv.R.p, lv.d_qoff.p, d_perm.p,
                                     lv.d_xoff.p, d_maxpiv.p, d_nonzero.p, lv.pts.p, lv.d_ranks.p, e, orth ? 1 : 0,
-                                    low ? 0 : 1, (int)nodes, (int)lv.maxM, st(), orth ? taus.p : nullptr),
+                                    (int)nodes, (int)lv.maxM, st()),
              "basis_finish");
         }
         if (orth) blocked_orth_qr<T>(lv, Rws.p, lv.Q.p, lv.R.p, taus.p, fixed_rank_rule(lv.dims, krows, e), low == nullptr);
@@ -1618,8 +1618,8 @@ class Solver : public SolverBase {
         Prof pfin("basis_finish", 0., (double)lv.qoff[nodes] * 24.);
         ck(launch_basis_finish<double>(lv.d_dims.p, d_krows.p, Rws.p, reinterpret_cast<double*>(lv.Q.p),
                                        reinterpret_cast<double*>(lv.R.p), lv.d_qoff.p, d_perm.p, lv.d_xoff.p,
-                                       d_maxpiv.p, d_nonzero.p, lv.pts.p, lv.d_ranks.p, e, 1, leaf ? 1 : 0,
-                                       (int)nodes, (int)lv.maxM, st(), taus.p),
+                                       d_maxpiv.p, d_nonzero.p, lv.pts.p, lv.d_ranks.p, e, 1,
+                                       (int)nodes, (int)lv.maxM, st()),
            "basis_finish");
       }
       blocked_orth_qr<double>(lv, Rws.p, reinterpret_cast<double*>(lv.Q.p), reinterpret_cast<double*>(lv.R.p),
@@ -1634,7 +1634,7 @@ class Solver : public SolverBase {
         Prof pfin("basis_finish", 0., (double)lv.qoff[nodes] * 24.);
         ck(launch_basis_finish<double>(lv.d_dims.p, d_krows.p, Rws.p, Qd.p, Rd.p, lv.d_qoff.p, d_perm.p,
                                        lv.d_xoff.p, d_maxpiv.p, d_nonzero.p, lv.pts.p, lv.d_ranks.p, e, 1,
-                                       leaf ? 1 : 0, (int)nodes, (int)lv.maxM, st(), taus.p),
+                                       (int)nodes, (int)lv.maxM, st()),
            "basis_finish");
       }
       blocked_orth_qr<double>(lv, Rws.p, Qd.p, Rd.p, taus.p, fixed_rank_rule(lv.dims, gram_krows, e), leaf);

@@ -6,10 +6,11 @@
 // shared memory and folded into R with Householder reflectors on
 // (row j of R, tile column j).  Step 2 (k_cpqr) runs the column-pivoted
 // Householder QR of R with Eigen 3.4's ColPivHouseholderQR pivot, norm
-// downdate and rank rules.  Step 3 (k_basis_finish) forms the interpolative
+// downdate and rank rules (in a cluster's shared memory where it fits,
+// k_cpqr.cu).  Step 3 (k_interp, k_basis_build) forms the interpolative
 // decomposition [I, R11^-1 R12], permutes the box bodies skeleton-first and
-// builds either the ID basis (operator mode) or the orthogonal basis with
-// completion plus the triangular R (preconditioner mode).
+// builds either the ID basis (operator mode) or, for the caller's orthogonal
+// completion, U_ID (preconditioner mode).
 #include "common.cuh"
 #include "kernels.h"
 
@@ -262,191 +263,147 @@ __global__ void __launch_bounds__(256) k_cpqr(const i64* __restrict__ dims, cons
   }
 }
 
-// Interpolative decomposition and the box basis.  W holds the packed CPQR
-// (row-major); Q (col-major, in/out) holds the incoming Q (identity at a
-// leaf, the children's R blocks above); R (col-major, out, zero on entry).
+// Rank rule and interpolation coefficients: T = R11^{-1} R12 in place (rows
+// 0..rank-1, columns rank..M-1 of the packed row-major factor in W).  One CTA
+// per box and 128 columns, a column per thread: back substitution by 32-row
+// blocks held in registers, R11 (scaled by the reciprocal pivots) staged in
+// shared memory so that a row block's multipliers come as 16-byte broadcasts.
+// Each element takes its updates from the last row upwards, unscaled, and is
+// divided by its pivot at the end, so the order of the operations does not
+// depend on the blocks.  Bound by FP64 FMA issue; with one barrier per row
+// and one CTA per box this was bound by the barriers (0.49 ms a level at 256
+// x 256 boxes of rank 128, whatever the number of boxes).
+constexpr int INTERP_NT = 128, INTERP_JT = 64;
+
 template <typename T>
-__global__ void __launch_bounds__(256) k_basis_finish(
-    const i64* __restrict__ dims, const i64* __restrict__ krows, T* __restrict__ Rws, T* __restrict__ Q,
-    T* __restrict__ Rm, const i64* __restrict__ qoff, const int* __restrict__ perm_in,
-    const i64* __restrict__ xoff, const double* __restrict__ maxpiv, const int* __restrict__ nonzero,
-    double* __restrict__ pts, i64* __restrict__ ranks_out, double epi, int orth, int qin_identity,
-    T* __restrict__ wy_taus, int xcap) {
-  const int box = blockIdx.x;
-  const int M = (int)dims[box];
-  const int K = (int)krows[box];
-  const int tid = threadIdx.x, nt = blockDim.x, lane = tid & 31, warp = tid >> 5, nw = nt >> 5;
-  if (M == 0 || K == 0) {
-    if (tid == 0) ranks_out[box] = 0;
+__global__ void __launch_bounds__(INTERP_NT) k_interp(const i64* __restrict__ dims, const i64* __restrict__ krows,
+                                                      T* __restrict__ Rws, const i64* __restrict__ qoff,
+                                                      const double* __restrict__ maxpiv,
+                                                      const int* __restrict__ nonzero, i64* __restrict__ ranks_out,
+                                                      double epi) {
+  constexpr int PS = 32 + 16 / sizeof(T);  // panel stride: 16-byte aligned columns, spread over the banks
+  const int box = blockIdx.x, tid = threadIdx.x;
+  const int M = (int)dims[box], K = (int)krows[box];
+  __shared__ __align__(16) T P[INTERP_JT * PS];  // P[j][i] = R11[b0 + i][j0 + j]
+  T* W = Rws + qoff[box];
+  int rank = 0;
+  if (M > 0 && K > 0) {
+    if (epi < 1.) {
+      const double thr = fabs(maxpiv[box]) * epi;
+      const int nz = nonzero[box];
+      for (int i0 = 0; i0 < nz; i0 += INTERP_NT) {
+        const int i = i0 + tid;
+        rank += __syncthreads_count(i < nz && fabs((double)W[(i64)i * M + i]) > thr);
+      }
+    } else {
+      rank = min(min(K, M), (int)floor(fmin(epi, 2147483647.)));
+    }
+  }
+  if (blockIdx.y == 0 && tid == 0) ranks_out[box] = rank;
+  if (!(0 < rank && rank < M)) return;
+  const int cb = rank + blockIdx.y * INTERP_NT;
+  if (cb >= M) return;
+  const int c = cb + tid;
+  const bool cv = c < M;
+  for (int b0 = (rank - 1) / 32 * 32; b0 >= 0; b0 -= 32) {
+    const int bs = min(32, rank - b0);
+    T r[32];
+#pragma unroll
+    for (int i = 0; i < 32; i++) r[i] = (cv && i < bs) ? W[(i64)(b0 + i) * M + c] : T(0);
+    // Columns from the last one down to the block's own triangle.
+    for (int je = rank; je > b0;) {
+      const bool diag = je <= b0 + 32;
+      const int jb = diag ? b0 : max(b0 + 32, je - INTERP_JT);
+      __syncthreads();
+      for (int e = tid; e < 32 * INTERP_JT; e += INTERP_NT) {
+        const int j = e % INTERP_JT, i = e / INTERP_JT;
+        T v = T(0);
+        if (i < bs && jb + j < je) v = W[(i64)(b0 + i) * M + jb + j] * (T(1) / W[(i64)(jb + j) * (M + 1)]);
+        P[j * PS + i] = v;
+      }
+      __syncthreads();
+      if (diag) break;
+      for (int j = je - 1; j >= jb; j -= 8) {
+        T x[8];
+#pragma unroll
+        for (int u = 0; u < 8; u++) x[u] = (cv && j - u >= jb) ? W[(i64)(j - u) * M + c] : T(0);
+#pragma unroll
+        for (int u = 0; u < 8; u++) {
+          if (j - u < jb) break;
+          const T* p = P + (j - u - jb) * PS;
+#pragma unroll
+          for (int i = 0; i < 32; i++) r[i] -= p[i] * x[u];
+        }
+      }
+      je = jb;
+    }
+#pragma unroll
+    for (int jj = 31; jj >= 0; jj--) {
+      if (jj >= bs) continue;
+      const T* p = P + jj * PS;
+#pragma unroll
+      for (int i = 0; i < jj; i++) r[i] -= p[i] * r[jj];
+    }
+    if (cv)
+#pragma unroll
+      for (int i = 0; i < 32; i++)
+        if (i < bs) W[(i64)(b0 + i) * M + c] = r[i];
+  }
+  if (cv)
+#pragma unroll 8
+    for (int i = 0; i < rank; i++) W[(i64)i * M + c] = W[(i64)i * M + c] / W[(i64)i * (M + 1)];
+}
+
+// The box basis from the interpolation coefficients, BASIS_COLS columns of a
+// box per CTA.  Q (col-major, in/out) holds the incoming Q (identity at a
+// leaf, the children's R blocks above); R (col-major, out, zero on entry).
+// Operator mode: Q = P [I; T^T], zero columns after, R = I.  Orthogonal mode:
+// U_ID = P [I; T^T] goes to R's slot and Q keeps the incoming Q (the caller
+// forms triu(Q) U_ID, its QR and Q).  The first CTA of a box also puts its
+// bodies in skeleton-first order.
+constexpr int BASIS_COLS = 32;
+
+template <typename T>
+__global__ void __launch_bounds__(256) k_basis_build(const i64* __restrict__ dims, const i64* __restrict__ krows,
+                                                     const T* __restrict__ Rws, T* __restrict__ Q, T* __restrict__ Rm,
+                                                     const i64* __restrict__ qoff, const int* __restrict__ perm_in,
+                                                     const i64* __restrict__ xoff, double* __restrict__ pts,
+                                                     const i64* __restrict__ ranks, int orth) {
+  const int box = blockIdx.x, tid = threadIdx.x, nt = blockDim.x;
+  const int M = (int)dims[box], i0 = blockIdx.y * BASIS_COLS;
+  if (M == 0 || krows[box] == 0 || i0 >= M) return;
+  const int rank = (int)ranks[box], w = min(BASIS_COLS, M - i0);
+  const T* W = Rws + qoff[box];
+  T* Qb = Q + qoff[box];
+  T* Rb = Rm + qoff[box];
+  if (!(0 < rank && rank < M)) {
+    // R = upper triangle of the incoming Q, Q = identity (h2matrix.cpp:57-60).
+    for_each_rc(M, w, [&](int r, int c, int) {
+      const i64 e = r + (i64)(i0 + c) * M;
+      Rb[e] = r <= i0 + c ? Qb[e] : T(0);
+      Qb[e] = r == i0 + c ? T(1) : T(0);
+    });
     return;
   }
   extern __shared__ __align__(16) unsigned char smem_raw[];
-  int* perm = reinterpret_cast<int*>(smem_raw);                          // M
-  double* sp = reinterpret_cast<double*>(smem_raw + ((4 * M + 15) / 16) * 16);  // 3M
-  T* taus = reinterpret_cast<T*>(sp + 3 * M);                            // M
-  __shared__ int s_rank;
-  __shared__ T s_red[32];
-  T* W = Rws + qoff[box];
-  T* Qb = Q + qoff[box];
-  T* Rb = Rm + qoff[box];
-  for (int c = tid; c < M; c += nt) perm[c] = perm_in[xoff[box] + c];
-  if (tid == 0) {
-    int size = K < M ? K : M;
-    int r = (int)floor(epi);
-    r = size < r ? size : r;
-    if (epi < 1.) {
-      double thr = fabs(maxpiv[box]) * epi;
-      r = 0;
-      for (int i = 0; i < nonzero[box]; i++) r += fabs((double)W[(i64)i * M + i]) > thr;
-    }
-    s_rank = r;
-  }
-  __syncthreads();
-  const int rank = s_rank;
-  if (!(0 < rank && rank < M)) {
-    // R = upper triangle of the incoming Q, Q = identity (h2matrix.cpp:57-60).
-    for_each_rc(M, M, [&](int r, int c, int e) {
-      Rb[e] = r <= c ? Qb[e] : T(0);
-    });
-    __syncthreads();
-    for_each_rc(M, M, [&](int r, int c, int e) {
-      Qb[e] = r == c ? T(1) : T(0);
-    });
-    if (tid == 0) ranks_out[box] = rank;
-    return;
-  }
-  // T = R11^{-1} R12 in place (rows 0..rank-1, columns rank..M-1), by
-  // column chunks staged in shared memory (as many columns as fit, so
-  // usually one chunk): back substitution with the whole CTA updating the
-  // rows above the current one (one barrier per row, one reciprocal of the
-  // pivot per row).
-  {
-    T* X = taus + M;  // rank x nc, row-major
-    const int nc = max(1, min(M - rank, xcap / rank));
-    for (int c0 = rank; c0 < M; c0 += nc) {
-      const int w = min(nc, M - c0);
-      for (int e = tid; e < rank * w; e += nt) X[e] = W[(i64)(e / w) * M + c0 + e % w];
-      __syncthreads();
-      for (int i = rank - 1; i >= 0; i--) {
-        const T inv = T(1) / W[(i64)i * M + i];
-        for (int k = warp; k < i; k += nw) {  // warp: row k, lanes: columns
-          const T wki = W[(i64)k * M + i] * inv;
-          for (int c = lane; c < w; c += 32) X[k * w + c] -= wki * X[i * w + c];
-        }
-        __syncthreads();
-      }
-      for (int e = tid; e < rank * w; e += nt) {
-        const int i = e / w;
-        W[(i64)i * M + c0 + e % w] = X[e] / W[(i64)i * M + i];
-      }
-      __syncthreads();
-    }
-  }
-  // Skeleton-first order of the box bodies.
+  int* perm = reinterpret_cast<int*>(smem_raw);                                 // M
+  double* sp = reinterpret_cast<double*>(smem_raw + ((4 * M + 15) / 16) * 16);  // 3 M
   double* bp = pts + 3 * xoff[box];
-  for (int e = tid; e < 3 * M; e += nt) sp[e] = bp[e];
+  for (int c = tid; c < M; c += nt) perm[c] = perm_in[xoff[box] + c];
+  if (i0 == 0)
+    for (int e = tid; e < 3 * M; e += nt) sp[e] = bp[e];
   __syncthreads();
-  for (int k = tid; k < M; k += nt) {
-    int p = perm[k];
-    bp[3 * k] = sp[3 * p];
-    bp[3 * k + 1] = sp[3 * p + 1];
-    bp[3 * k + 2] = sp[3 * p + 2];
-  }
-  if (!orth) {
-    // Q = P [I; T^T] padded with zero columns, R = I (h2matrix.cpp:50-55).
-    for (i64 e = tid; e < (i64)M * M; e += nt) Qb[e] = T(0);
-    __syncthreads();
-    for_each_rc(M, rank, [&](int k, int i, int e) {
-      T v = k < rank ? (k == i ? T(1) : T(0)) : W[(i64)i * M + k];
-      Qb[(i64)perm[k] + (i64)i * M] = v;
-    });
-    for (int i = tid; i < rank; i += nt) Rb[(i64)i * M + i] = T(1);
-    if (tid == 0) ranks_out[box] = rank;
-    return;
-  }
-  // Orthogonal mode (h2matrix.cpp:43-49).  U_ID = P [I; T^T] (M x rank)
-  // goes to R's slot as scratch, RX2 = triu(Qin) U_ID to W (col-major now).
-  for_each_rc(M, rank, [&](int k, int i, int e) {
-    T v = k < rank ? (k == i ? T(1) : T(0)) : W[(i64)i * M + k];
-    Rb[(i64)perm[k] + (i64)i * M] = v;
+  if (i0 == 0)
+    for (int e = tid; e < 3 * M; e += nt) bp[e] = sp[3 * perm[e / 3] + e % 3];
+  T* out = orth ? Rb : Qb;
+  for_each_rc(M, orth ? min(w, rank - i0) : w, [&](int k, int c, int) {
+    const int i = i0 + c;
+    T v = T(0);
+    if (i < rank) v = k < rank ? (k == i ? T(1) : T(0)) : W[(i64)i * M + k];
+    out[(i64)perm[k] + (i64)i * M] = v;
   });
-  __syncthreads();
-  if (wy_taus) {
-    // Blocked completion on the host side: U_ID is in R's slot, Q still
-    // holds Q_in; the caller forms triu(Q_in) U_ID, its QR and Q.
-    if (tid == 0) ranks_out[box] = rank;
-    return;
-  }
-  for_each_rc(M, rank, [&](int p, int i, int e) {
-    T s;
-    if (qin_identity) {
-      s = Rb[e];
-    } else {
-      s = 0;
-      for (int l = p; l < M; l++) s += Qb[p + (i64)l * M] * Rb[l + (i64)i * M];
-    }
-    W[e] = s;
-  });
-  __syncthreads();
-  // Householder QR of RX2 (M x rank), column-major in W.  One warp per
-  // column for the reflector application.
-  for (int k = 0; k < rank; k++) {
-    T* colk = W + (i64)k * M;
-    T part = 0;
-    for (int r = k + 1 + tid; r < M; r += nt) part += colk[r] * colk[r];
-    T tsq = BlockReduce<T>::sum(part, s_red);
-    T c0 = colk[k];
-    T tau = 0, beta = c0, scale = 0;
-    if (tsq > Tiny<T>::v()) {
-      beta = sqrt(c0 * c0 + tsq);
-      if (c0 >= T(0)) beta = -beta;
-      scale = T(1) / (c0 - beta);
-      tau = (beta - c0) / beta;
-    }
-    __syncthreads();
-    for (int r = k + 1 + tid; r < M; r += nt) colk[r] *= scale;
-    if (tid == 0) {
-      colk[k] = beta;
-      taus[k] = tau;
-    }
-    __syncthreads();
-    if (tau != T(0))
-      for (int j = k + 1 + warp; j < rank; j += nw) {
-        T* colj = W + (i64)j * M;
-        T w = 0;
-        for (int r = k + 1 + lane; r < M; r += 32) w += colk[r] * colj[r];
-        for (int o = 16; o > 0; o >>= 1) w += __shfl_xor_sync(0xffffffffu, w, o);
-        w = (w + colj[k]) * tau;
-        if (lane == 0) colj[k] -= w;
-        for (int r = k + 1 + lane; r < M; r += 32) colj[r] -= w * colk[r];
-      }
-    __syncthreads();
-  }
-  // R = triu(RX2[:rank, :rank]) (R's slot was scratch: clear first).
-  for_each_rc(M, M, [&](int r, int c, int e) {
-    Rb[e] = (c < rank && r <= c) ? W[r + (i64)c * M] : T(0);
-  });
-  // Q = H_0 ... H_{rank-1} applied to the identity.
-  for_each_rc(M, M, [&](int r, int c, int e) {
-    Qb[e] = r == c ? T(1) : T(0);
-  });
-  __syncthreads();
-  for (int k = rank - 1; k >= 0; k--) {
-    const T tau = taus[k];
-    const T* colk = W + (i64)k * M;
-    if (tau != T(0))
-      for (int j = k + warp; j < M; j += nw) {
-        T* qj = Qb + (i64)j * M;
-        T w = 0;
-        for (int r = k + 1 + lane; r < M; r += 32) w += colk[r] * qj[r];
-        for (int o = 16; o > 0; o >>= 1) w += __shfl_xor_sync(0xffffffffu, w, o);
-        w = (w + qj[k]) * tau;
-        if (lane == 0) qj[k] -= w;
-        for (int r = k + 1 + lane; r < M; r += 32) qj[r] -= w * colk[r];
-      }
-    __syncthreads();
-  }
-  if (tid == 0) ranks_out[box] = rank;
+  if (!orth)
+    for (int i = i0 + tid; i < min(i0 + w, rank); i += nt) Rb[(i64)i * M + i] = T(1);
 }
 
 // ---------------------------------------------------------------- launchers
@@ -471,8 +428,19 @@ cudaError_t launch_sample_tsqr(const KernelParams& kp, const double* bodies, con
 
 template <typename T>
 cudaError_t launch_cpqr(const i64* dims, const i64* krows, T* Rws, const i64* qoff, int* perm, const i64* xoff,
-                        double* maxpiv, int* nonzero, i64 step_cap, int nboxes, int maxM, cudaStream_t st) {
+                        double* maxpiv, int* nonzero, i64 step_cap, double epi, int nboxes, int maxM, cudaStream_t st) {
   if (nboxes == 0) return cudaSuccess;
+  // Threshold (operator) bases whose matrix fits the shared memory of a
+  // cluster.  Fixed-rank ones keep k_cpqr and its order of the sums: they are
+  // formed here only in the mode that follows the reference's own sequence,
+  // whose factorization amplifies the rounding of the bases to percents on the
+  // ill-conditioned reference configuration.
+  if (step_cap < 0) {
+    bool done = false;
+    const cudaError_t e = launch_cpqr_cluster<T>(dims, krows, Rws, qoff, perm, xoff, maxpiv, nonzero, 0.5 * epi,
+                                                 nboxes, maxM, st, &done);
+    if (e != cudaSuccess || done) return e;
+  }
   size_t smem = 2 * sizeof(double) * maxM + sizeof(T) * maxM + sizeof(int) * maxM + 64;
   auto fn = k_cpqr<T>;
   cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
@@ -485,19 +453,20 @@ cudaError_t launch_cpqr(const i64* dims, const i64* krows, T* Rws, const i64* qo
 template <typename T>
 cudaError_t launch_basis_finish(const i64* dims, const i64* krows, T* Rws, T* Q, T* R, const i64* qoff,
                                 const int* perm, const i64* xoff, const double* maxpiv, const int* nonzero,
-                                double* pts, i64* ranks, double epi, int orth, int qin_identity, int nboxes,
-                                int maxM, cudaStream_t st, T* wy_taus) {
+                                double* pts, i64* ranks, double epi, int orth, int nboxes, int maxM,
+                                cudaStream_t st) {
   if (nboxes == 0) return cudaSuccess;
-  // Back-substitution chunk: columns of rank rows, at most 96 KB (all
-  // M - rank columns of a 256-box at rank >= 64 in FP64).
-  const int xcap = (int)std::min<size_t>((size_t)maxM * maxM, 96 * 1024 / sizeof(T));
-  size_t smem = ((4 * (size_t)maxM + 15) / 16) * 16 + sizeof(double) * 3 * maxM + sizeof(T) * (maxM + xcap) + 64;
-  auto fn = k_basis_finish<T>;
-  cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  note_launch();
+  k_interp<T><<<dim3(nboxes, (maxM + INTERP_NT - 1) / INTERP_NT), INTERP_NT, 0, st>>>(dims, krows, Rws, qoff, maxpiv,
+                                                                                      nonzero, ranks, epi);
+  cudaError_t e = cudaGetLastError();
+  if (e != cudaSuccess) return e;
+  const size_t smem = ((4 * (size_t)maxM + 15) / 16) * 16 + sizeof(double) * 3 * maxM;
+  e = cudaFuncSetAttribute(k_basis_build<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (e != cudaSuccess) return e;
   note_launch();
-  fn<<<nboxes, 256, smem, st>>>(dims, krows, Rws, Q, R, qoff, perm, xoff, maxpiv, nonzero, pts, ranks, epi, orth,
-                                qin_identity, wy_taus, xcap);
+  k_basis_build<T><<<dim3(nboxes, (maxM + BASIS_COLS - 1) / BASIS_COLS), 256, smem, st>>>(
+      dims, krows, Rws, Q, R, qoff, perm, xoff, pts, ranks, orth);
   return cudaGetLastError();
 }
 
@@ -506,10 +475,10 @@ cudaError_t launch_basis_finish(const i64* dims, const i64* krows, T* Rws, T* Q,
                                              const i64*, const int*, const i64*, T*, const i64*, int, int,       \
                                              cudaStream_t);                                                       \
   template cudaError_t launch_cpqr<T>(const i64*, const i64*, T*, const i64*, int*, const i64*, double*, int*,    \
-                                      i64, int, int, cudaStream_t);                                               \
+                                      i64, double, int, int, cudaStream_t);                                       \
   template cudaError_t launch_basis_finish<T>(const i64*, const i64*, T*, T*, T*, const i64*, const int*,         \
                                               const i64*, const double*, const int*, double*, i64*, double, int,  \
-                                              int, int, int, cudaStream_t, T*);
+                                              int, int, cudaStream_t);
 INST(double)
 INST(float)
 #undef INST
@@ -548,7 +517,7 @@ namespace h2b {
 // squared column norm a column-pivoted QR of XF would pick), so pivots and
 // rows of R equal those of ColPivHouseholderQR in exact arithmetic
 // (h2matrix.cpp:27); R goes to Rws row-major in pivoted column order, where
-// k_cpqr leaves it, for k_basis_finish.  Once the Schur diagonal falls to
+// k_cpqr leaves it, for k_interp.  Once the Schur diagonal falls to
 // rounding noise of the FP64 Gram matrix (16 eps max diag), the pivots
 // still to be taken get the row [floor, 0, ..., 0] with floor =
 // sqrt(eps max diag): their interpolation coefficients come out exactly zero.
@@ -768,7 +737,7 @@ namespace h2b {
 
 // One Householder panel of the M x rank matrix W (column-major, ld M) of a
 // box: columns k0..k0+nb-1, rows k0..M-1, factored in shared memory with the
-// same reflector convention as k_basis_finish (beta = -sign(c0) * norm).
+// same reflector convention as the reference (beta = -sign(c0) * norm).
 // Writes back R (upper) and the reflector tails (lower), the explicit unit
 // lower-trapezoidal V of the panel to Vp ((M-k0) x nb), the panel's
 // compact-WY T (nb x nb, I - V T V^T = H_k0 ... H_k0+nb-1) to Tp and its

@@ -42,12 +42,20 @@ int sketch_tile_rows();
 int sketch_tile_cols();
 template <typename T>
 cudaError_t launch_cpqr(const i64* dims, const i64* krows, T* Rws, const i64* qoff, int* perm, const i64* xoff,
-                        double* maxpiv, int* nonzero, i64 step_cap, int nboxes, int maxM, cudaStream_t st);
+                        double* maxpiv, int* nonzero, i64 step_cap, double epi, int nboxes, int maxM, cudaStream_t st);
+// k_cpqr.cu: one cluster per box; *launched stays false where a box of maxM
+// columns does not fit a cluster's shared memory.
+template <typename T>
+cudaError_t launch_cpqr_cluster(const i64* dims, const i64* krows, T* Rws, const i64* qoff, int* perm,
+                                const i64* xoff, double* maxpiv, int* nonzero, double stop_rel, int nboxes,
+                                int maxM, cudaStream_t st, bool* launched);
+// Rank, interpolation and basis of every box (k_interp, k_basis_build); orth:
+// U_ID is left in R's slot and Q keeps the incoming Q.
 template <typename T>
 cudaError_t launch_basis_finish(const i64* dims, const i64* krows, T* Rws, T* Q, T* R, const i64* qoff,
                                 const int* perm, const i64* xoff, const double* maxpiv, const int* nonzero,
-                                double* pts, i64* ranks, double epi, int orth, int qin_identity, int nboxes,
-                                int maxM, cudaStream_t st, T* wy_taus = nullptr);
+                                double* pts, i64* ranks, double epi, int orth, int nboxes, int maxM,
+                                cudaStream_t st);
 // Compact-WY T matrix per box (see k_wy_t).
 template <typename T>
 struct WyTask {

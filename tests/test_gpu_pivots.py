@@ -1,0 +1,56 @@
+"""The pivoted factorizations of a box at the sizes where their kernels change:
+the LU of a redundant block (panel, register-row and shared-memory limits) and
+the column-pivoted QR of an operator box (cluster sizes, rows per lane, the
+kernel for boxes beyond a cluster)."""
+import numpy as np
+import pytest
+
+import h2_oracle as O
+import mxc_b200 as m
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("precision", [m.FP64, m.FP32])
+@pytest.mark.parametrize("n", [1, 2, 31, 32, 33, 64, 95, 146, 147, 203, 204, 256, 257, 512, 513, 1024, 1025])
+def test_single_box_solve_is_backward_stable(handle, n, precision):
+    """A tree of one box has rank 0: factorize is the partial-pivot LU of the
+    dense matrix and solvePrecondition its solve.  The small diagonal makes the
+    rows move.  The residual is within the LU's backward error, about
+    eps n growth ||K|| ||x|| (growth at most about n^(2/3) in practice)."""
+    b = np.random.default_rng(n).random((n, 3))
+    t = m.build_tree(b, 0)
+    M = m.H2MatrixSolver(handle, m.Laplace3D(10.0), 0.0, 8, 0, t, 2.0, b, precision=precision)
+    assert M.factorizeM() == [0]
+    rhs = np.asfortranarray(np.random.default_rng(1).random((n, 3)))
+    x = rhs.copy(order="F")
+    M.solvePrecondition(x)
+    K = O.gen_matrix(O.Kernel(O.LAPLACE, 10.0), b, b)
+    eps = np.finfo(np.float64 if precision == m.FP64 else np.float32).eps
+    bound = eps * n ** (2.0 / 3.0) * 10 * np.linalg.norm(K) * np.linalg.norm(x) + eps * np.linalg.norm(rhs)
+    assert np.linalg.norm(K @ x - rhs) < bound
+
+
+@pytest.mark.parametrize("box", [20, 33, 156, 157, 256, 257, 312, 480, 513, 650, 769])
+@pytest.mark.parametrize("eps", [1e-3, 1e-9])
+def test_operator_box_sizes(handle, box, eps):
+    """Operators whose leaves hold `box` bodies: the product is within ten
+    times the bases' threshold of the dense one, and the interpolation keeps
+    every body (the skeleton order is a permutation)."""
+    n = 8 * box
+    b = np.random.default_rng(box).random((n, 3))
+    t = m.build_tree(b, 3)
+    k = m.Laplace3D(1e-2)
+    A = m.H2MatrixSolver(handle, k, eps, 100, 0, t, 1.0, b)
+    dims, ranks = A.level_dims(3)
+    assert np.all(ranks > 0) and np.all(ranks <= dims)
+    S = A.export(3, m._lib.EXPORT_S).reshape(-1, 3)
+    for i in range(8):
+        own = b[i * box:(i + 1) * box]
+        got = S[i * box:(i + 1) * box]
+        assert np.array_equal(got[np.lexsort(got.T)], own[np.lexsort(own.T)])
+    x = np.random.default_rng(2).random(n)
+    y = x.copy()
+    A.matVecMul(y)
+    d = m.dense_matvec(handle, k, b, x)
+    assert np.linalg.norm(y - d) < 10 * eps * np.linalg.norm(d)

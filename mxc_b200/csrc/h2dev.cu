@@ -1583,33 +1583,10 @@ class Solver : public SolverBase {
       DVec<double> state;
       d_steps.upload(steps);
       state.alloc(3 * nodes);
-      // The trailing-update plans depend only on the sizes: all are built
-      // (and uploaded) before the first panel, so the device does not wait
-      // for host planning between panels.
-      std::vector<GemmPlan<double>> ups;
-      ups.reserve((size_t)std::max<i64>(0, (maxsteps - 1) / nb));
-      for (i64 k0 = 0; k0 + nb < maxsteps; k0 += nb) {
-        const i64 k1 = k0 + nb;
-        ups.emplace_back();
-        GemmPlan<double>& up = ups.back();
-        up.name = "gemm_pivchol_update";
-        for (i64 i = 0; i < nodes; i++) {
-          const i64 M = lv.dims[i];
-          if (steps[i] <= k1 || M <= k1) continue;
-          double* Rb = Rws.p + lv.qoff[i];
-          up.add_task(G.p + lv.qoff[i] + k1 + k1 * M, M, (int)(M - k1), (int)(M - k1), 1.);
-          up.add_entry(Rb + k0 * M + k1, M, 0, Rb + k0 * M + k1, M, 1, nb, -1.);
-        }
-        up.finalize();
-      }
       Prof pf("pivchol", fl, 0.);
-      for (i64 k0 = 0, p = 0; k0 < maxsteps; k0 += nb, p++) {
-        ck(launch_pivchol_panel(lv.d_dims.p, d_steps.p, G.p, Rws.p, lv.d_qoff.p, d_perm.p, lv.d_xoff.p, state.p,
-                                (int)k0, nb, (int)nodes, (int)lv.maxM, st()),
-           "pivchol panel");
-        if (k0 + nb >= maxsteps) break;
-        ups[p].run(st());
-      }
+      ck(launch_pivchol(lv.d_dims.p, d_steps.p, G.p, Rws.p, lv.d_qoff.p, d_perm.p, lv.d_xoff.p, state.p, (int)maxsteps,
+                        (int)nodes, (int)lv.maxM, st()),
+         "pivchol");
     }
     DVec<double> taus;
     taus.alloc(std::max<i64>(1, lv.lenX));

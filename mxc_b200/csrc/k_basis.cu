@@ -511,127 +511,292 @@ cudaError_t launch_gather_points(const double* bodies, const int* idx, i64 n, do
 
 namespace h2b {
 
-// One 32-pivot panel of the blocked pivoted Cholesky of the Gram matrix
-// G = XF^T XF (M x M per box, symmetric), stopped after ``steps`` pivots in
-// all.  The pivot is the largest remaining Schur-complement diagonal (the
-// squared column norm a column-pivoted QR of XF would pick), so pivots and
-// rows of R equal those of ColPivHouseholderQR in exact arithmetic
-// (h2matrix.cpp:27); R goes to Rws row-major in pivoted column order, where
-// k_cpqr leaves it, for k_interp.  Once the Schur diagonal falls to
-// rounding noise of the FP64 Gram matrix (16 eps max diag), the pivots
-// still to be taken get the row [floor, 0, ..., 0] with floor =
-// sqrt(eps max diag): their interpolation coefficients come out exactly zero.
-// G already carries the trailing updates of earlier panels; this panel's
-// pivots are taken left-looking: the Schur diagonal of the remaining
-// columns lives in shared memory and loses R[k][j]^2 after every pivot, and
-// row k of R is G[k][j] minus the panel's earlier rows.  The caller applies
-// G_trail -= R_panel^T R_panel (one batched GEMM) afterwards.
-__global__ void __launch_bounds__(256) k_pivchol_panel(const i64* __restrict__ dims, const i64* __restrict__ steps_box,
-                                                       double* __restrict__ G, double* __restrict__ Rws,
-                                                       const i64* __restrict__ qoff, int* __restrict__ perm_g,
-                                                       const i64* __restrict__ xoff, double* __restrict__ state,
-                                                       int k0, int nb) {
+// Blocked pivoted Cholesky of the Gram matrix G = XF^T XF (M x M per box,
+// symmetric), stopped after ``steps`` pivots: the largest remaining Schur
+// diagonal (the squared column norm a column-pivoted QR of XF would pick) is
+// the pivot, so pivots and rows of R equal those of ColPivHouseholderQR in
+// exact arithmetic (h2matrix.cpp:27).  Once the Schur diagonal falls to
+// rounding noise of the FP64 Gram matrix (16 eps max diag), the pivots still to
+// be taken get the row [floor, 0, ..., 0] with floor = sqrt(eps max diag):
+// their interpolation coefficients come out exactly zero.
+//
+// k_pivchol_panel takes up to PC_NB pivots left-looking: row k of R is G's row
+// of the pivot minus the panel's earlier rows, and the Schur diagonal loses
+// R[k][j]^2.  Columns never move: thread j keeps its columns' position in the
+// pivoted order (exchanged as swaps would) and their Schur diagonal in
+// registers, the panel's rows of R are in shared memory (SM; in R itself for
+// boxes too wide), and a pivot costs one barrier, the read of G's row from L2
+// and the chain of the panel's rows.  k_pivchol_update subtracts
+// R_panel^T R_panel from all of G, on the FP64 tensor cores (finished columns
+// too: nothing reads those).  The panel that takes the last pivot puts R's rows
+// in pivoted order, where k_cpqr leaves them, and writes perm.
+//
+// Bound: the latency of that chain, about 1.5 us a pivot.  With the rows and
+// columns of G and R exchanged in memory and four barriers a pivot it was 5 us
+// (0.6 ms a level of 128 pivots for 1 to 128 boxes), and the updates, planned on
+// the host as GEMMs of the shrinking trailing blocks, left gaps of 0.5 ms a
+// level: 65,536 bodies, nine levels, 5.8 -> 2.4 ms of kernels.
+constexpr int PC_NB = 32, PC_NT = 256, PC_T = 64;
+
+__device__ __forceinline__ unsigned long long pc_key(double v) {
+  // Larger value, larger key; values not above -1 and NaN have key 0.
+  if (!(v > -1.)) return 0ULL;
+  const unsigned long long u = (unsigned long long)__double_as_longlong(v);
+  return (u >> 63) ? ~u : (u | 0x8000000000000000ULL);
+}
+__device__ __forceinline__ double pc_value(unsigned long long key) {
+  return __longlong_as_double((long long)((key >> 63) ? (key & 0x7fffffffffffffffULL) : ~key));
+}
+// Warp-wide largest key, and the smallest tag that has it.
+__device__ __forceinline__ void pc_warp_best(unsigned long long& key, unsigned& tag) {
+  const unsigned hi = (unsigned)(key >> 32), m = __reduce_max_sync(0xffffffffu, hi);
+  const unsigned lo = __reduce_max_sync(0xffffffffu, hi == m ? (unsigned)key : 0u);
+  const unsigned long long best = ((unsigned long long)m << 32) | lo;
+  tag = __reduce_min_sync(0xffffffffu, key == best ? tag : 0xffffffffu);
+  key = best;
+}
+
+template <int CPT, bool SM>
+__global__ void __launch_bounds__(PC_NT) k_pivchol_panel(const i64* __restrict__ dims,
+                                                         const i64* __restrict__ steps_box, const double* __restrict__ G,
+                                                         double* __restrict__ Rws, const i64* __restrict__ qoff,
+                                                         int* __restrict__ perm_g, const i64* __restrict__ xoff,
+                                                         double* __restrict__ state, int k0) {
+  constexpr int NW = PC_NT / 32;
   const int box = blockIdx.x;
   const int M = (int)dims[box];
   const int steps = (int)steps_box[box];
   if (M == 0 || k0 >= steps) return;
   extern __shared__ __align__(16) unsigned char smem_raw[];
-  double* dsch = reinterpret_cast<double*>(smem_raw);  // M
-  __shared__ double red_v[32];
-  __shared__ int red_i[32];
-  double* g = G + qoff[box];
+  __shared__ unsigned long long s_key[2][NW];
+  __shared__ unsigned s_tag[2][NW];
+  const double* g = G + qoff[box];
   double* R = Rws + qoff[box];
-  int* perm = perm_g + xoff[box];
+  double* Rp = SM ? reinterpret_cast<double*>(smem_raw) : R + (i64)k0 * M;  // the panel's rows, ld M
+  int* perm = perm_g + xoff[box];  // positions of the columns until the last panel
   double* st = state + 3 * (i64)box;  // [rfloor, noise threshold, noise flag]
-  const int tid = threadIdx.x, nt = blockDim.x;
-  if (k0 == 0) {
-    for (int c = tid; c < M; c += nt) perm[c] = c;
-    double dmax = 0.;
-    int dmi = 0;
-    for (int j = tid; j < M; j += nt) {
-      double v = g[(i64)j * M + j];
-      if (v > dmax) { dmax = v; dmi = j; }
-    }
-    argmax_first(dmax, dmi, red_v, red_i);
-    if (tid == 0) {
-      double rf = sqrt(DBL_EPSILON * dmax);
-      st[0] = rf > 0. ? rf : DBL_MIN;
-      st[1] = 16. * DBL_EPSILON * dmax;
-      st[2] = 0.;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  // Best own column not yet taken, over the whole box; b: buffer.
+  auto best = [&](unsigned long long& key, unsigned& tag, int b) {
+    pc_warp_best(key, tag);
+    if (lane == 0) {
+      s_key[b][warp] = key;
+      s_tag[b][warp] = tag;
     }
     __syncthreads();
+    key = lane < NW ? s_key[b][lane] : 0ULL;
+    tag = lane < NW ? s_tag[b][lane] : 0xffffffffu;
+    pc_warp_best(key, tag);
+  };
+  int pos[CPT];
+  double dsch[CPT];
+#pragma unroll
+  for (int u = 0; u < CPT; u++) {
+    const int j = tid + u * PC_NT;
+    pos[u] = j >= M ? -1 : k0 == 0 ? j : perm[j];
+    dsch[u] = pos[u] >= k0 ? g[(i64)j * M + j] : 0.;
   }
-  const double rfloor = st[0], noise = st[1];
-  bool noise_mode = st[2] != 0.;
-  for (int j = tid; j < M; j += nt) dsch[j] = j >= k0 ? g[(i64)j * M + j] : 0.;
-  __syncthreads();
-  const int kend = (k0 + nb < steps) ? k0 + nb : steps;
-  for (int k = k0; k < kend; k++) {
-    double bv = -1.;
-    int bi = 0x7fffffff;
-    for (int j = k + tid; j < M; j += nt)
-      if (dsch[j] > bv) { bv = dsch[j]; bi = j; }
-    argmax_first(bv, bi, red_v, red_i);
-    if (bi < k || bi >= M) bi = k;
-    if (bi != k) {
-      // Rows/columns k0.. of G are the live trailing matrix; earlier rows of
-      // R (all panels) follow the column exchange.
-      for (int c = k0 + tid; c < M; c += nt) {
-        double t = g[(i64)k * M + c];
-        g[(i64)k * M + c] = g[(i64)bi * M + c];
-        g[(i64)bi * M + c] = t;
-      }
-      __syncthreads();
-      for (int r = k0 + tid; r < M; r += nt) {
-        double t = g[(i64)r * M + k];
-        g[(i64)r * M + k] = g[(i64)r * M + bi];
-        g[(i64)r * M + bi] = t;
-      }
-      for (int r = tid; r < k; r += nt) {
-        double t = R[(i64)r * M + k];
-        R[(i64)r * M + k] = R[(i64)r * M + bi];
-        R[(i64)r * M + bi] = t;
-      }
-      if (tid == 0) {
-        double t = dsch[k]; dsch[k] = dsch[bi]; dsch[bi] = t;
-        int ti = perm[k]; perm[k] = perm[bi]; perm[bi] = ti;
-      }
+  double rfloor, noise;
+  bool noise_mode = false;
+  if (k0 == 0) {
+    unsigned long long key = 0;
+    unsigned tag = 0;
+#pragma unroll
+    for (int u = 0; u < CPT; u++)
+      if (pos[u] >= 0 && dsch[u] > 0. && pc_key(dsch[u]) > key) key = pc_key(dsch[u]);
+    best(key, tag, 1);
+    const double dmax = key ? pc_value(key) : 0.;
+    const double rf = sqrt(DBL_EPSILON * dmax);
+    rfloor = rf > 0. ? rf : DBL_MIN;
+    noise = 16. * DBL_EPSILON * dmax;
+    if (tid == 0) {
+      st[0] = rfloor;
+      st[1] = noise;
     }
-    __syncthreads();
-    const double d = dsch[k];
+  } else {
+    rfloor = st[0];
+    noise = st[1];
+    noise_mode = st[2] != 0.;
+  }
+  const int kend = (k0 + PC_NB < steps) ? k0 + PC_NB : steps;
+  for (int k = k0; k < kend; k++) {
+    unsigned long long key = 0;
+    unsigned tag = 0xffffffffu;  // position << 16 | column
+#pragma unroll
+    for (int u = 0; u < CPT; u++)
+      if (pos[u] >= k) {
+        const unsigned long long ku = pc_key(dsch[u]);
+        const unsigned tu = ((unsigned)pos[u] << 16) | (unsigned)(tid + u * PC_NT);
+        if (ku > key || (ku == key && tu < tag)) { key = ku; tag = tu; }
+      }
+    best(key, tag, (k - k0) & 1);
+    const int p = (int)(tag >> 16), pc = (int)(tag & 0xffffu);
+    double d = key ? pc_value(key) : __longlong_as_double(0x7ff8000000000000LL);
     if (!(d > noise)) noise_mode = true;
-    if (noise_mode) {
-      for (int j = k + tid; j < M; j += nt) R[(i64)k * M + j] = (j == k) ? rfloor : 0.;
-      __syncthreads();
-      continue;
+    double v[CPT];
+    if (!noise_mode) {
+#pragma unroll
+      for (int u = 0; u < CPT; u++) {
+        const int j = tid + u * PC_NT;
+        v[u] = j < M ? g[(i64)pc * M + j] : 0.;
+      }
     }
     const double rkk = sqrt(d);
     const double inv = 1. / rkk;
-    for (int j = k + tid; j < M; j += nt) {
-      double v;
-      if (j == k) {
-        v = rkk;
-      } else {
-        v = g[(i64)k * M + j];
-        for (int p = k0; p < k; p++) v -= R[(i64)p * M + k] * R[(i64)p * M + j];
-        v *= inv;
-        dsch[j] -= v * v;
-      }
-      R[(i64)k * M + j] = v;
+#pragma unroll
+    for (int u = 0; u < CPT; u++) {
+      const int j = tid + u * PC_NT;
+      if (j == pc)
+        pos[u] = k;
+      else if (pos[u] == k)
+        pos[u] = p;
     }
-    __syncthreads();
+    if (noise_mode) {
+#pragma unroll
+      for (int u = 0; u < CPT; u++)
+        if (pos[u] >= k) v[u] = pos[u] == k ? rfloor : 0.;
+    } else {
+#pragma unroll 8
+      for (int i = 0; i < k - k0; i++) {
+        const double m = Rp[(size_t)i * M + pc];
+#pragma unroll
+        for (int u = 0; u < CPT; u++) {
+          const int j = tid + u * PC_NT;
+          if (j < M) v[u] -= m * Rp[(size_t)i * M + j];
+        }
+      }
+#pragma unroll
+      for (int u = 0; u < CPT; u++) {
+        if (pos[u] == k) {
+          v[u] = rkk;
+        } else {
+          v[u] *= inv;
+          dsch[u] -= v[u] * v[u];
+        }
+      }
+    }
+#pragma unroll
+    for (int u = 0; u < CPT; u++) {
+      const int j = tid + u * PC_NT;
+      if (j >= M) continue;
+      const double x = pos[u] >= k ? v[u] : 0.;
+      if (SM) Rp[(size_t)(k - k0) * M + j] = x;
+      R[(i64)k * M + j] = x;
+    }
+    if (!SM) __threadfence_block();
   }
   if (tid == 0) st[2] = noise_mode ? 1. : 0.;
+  if (kend < steps) {
+#pragma unroll
+    for (int u = 0; u < CPT; u++)
+      if (pos[u] >= 0) perm[tid + u * PC_NT] = pos[u];
+    return;
+  }
+  // Last panel: the rows in pivoted order, eight at a time.
+  __syncthreads();
+  for (int k = 0; k < steps; k += 8) {
+    double v[8][CPT];
+#pragma unroll
+    for (int i = 0; i < 8; i++)
+#pragma unroll
+      for (int u = 0; u < CPT; u++)
+        v[i][u] = (k + i < steps && pos[u] >= 0) ? R[(i64)(k + i) * M + tid + u * PC_NT] : 0.;
+    __syncthreads();
+#pragma unroll
+    for (int i = 0; i < 8; i++)
+#pragma unroll
+      for (int u = 0; u < CPT; u++)
+        if (k + i < steps && pos[u] >= 0) R[(i64)(k + i) * M + pos[u]] = v[i][u];
+  }
+#pragma unroll
+  for (int u = 0; u < CPT; u++)
+    if (pos[u] >= 0) perm[pos[u]] = tid + u * PC_NT;
 }
 
-cudaError_t launch_pivchol_panel(const i64* dims, const i64* steps_box, double* G, double* Rws, const i64* qoff,
-                                 int* perm, const i64* xoff, double* state, int k0, int nb, int nboxes, int maxM,
-                                 cudaStream_t st) {
+// G -= R_panel^T R_panel for one 64 x 64 tile of one box: mma.sync m8n8k4,
+// four warps of 32 x 32.
+__global__ void __launch_bounds__(128) k_pivchol_update(const i64* __restrict__ dims,
+                                                        const i64* __restrict__ steps_box, double* __restrict__ G,
+                                                        const double* __restrict__ Rws, const i64* __restrict__ qoff,
+                                                        int k0) {
+  constexpr int LD = PC_T + 4;
+  const int box = blockIdx.x, M = (int)dims[box], steps = (int)steps_box[box];
+  const int nt = (M + PC_T - 1) / PC_T, r0 = (int)blockIdx.y / nt * PC_T, c0 = (int)blockIdx.y % nt * PC_T;
+  if (M == 0 || k0 + PC_NB >= steps || r0 >= M) return;  // no pivot left to take
+  __shared__ double As[PC_NB][LD], Bs[PC_NB][LD];
+  const double* R = Rws + qoff[box] + (i64)k0 * M;
+  double* g = G + qoff[box];
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, wm = warp >> 1, wn = warp & 1;
+  const int fr = lane >> 2, fk = lane & 3;
+  for (int e = tid; e < PC_NB * PC_T; e += 128) {
+    const int i = e / PC_T, j = e % PC_T;
+    As[i][j] = r0 + j < M ? -R[(i64)i * M + r0 + j] : 0.;
+    Bs[i][j] = c0 + j < M ? R[(i64)i * M + c0 + j] : 0.;
+  }
+  __syncthreads();
+  double acc[4][4][2];
+#pragma unroll
+  for (int i = 0; i < 4; i++)
+#pragma unroll
+    for (int j = 0; j < 4; j++) acc[i][j][0] = acc[i][j][1] = 0.;
+#pragma unroll
+  for (int ks = 0; ks < PC_NB; ks += 4) {
+    double a[4], b[4];
+#pragma unroll
+    for (int i = 0; i < 4; i++) a[i] = As[ks + fk][wm * 32 + i * 8 + fr];
+#pragma unroll
+    for (int j = 0; j < 4; j++) b[j] = Bs[ks + fk][wn * 32 + j * 8 + fr];
+#pragma unroll
+    for (int i = 0; i < 4; i++)
+#pragma unroll
+      for (int j = 0; j < 4; j++)
+        asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0, %1}, {%2}, {%3}, {%0, %1};\n"
+                     : "+d"(acc[i][j][0]), "+d"(acc[i][j][1])
+                     : "d"(a[i]), "d"(b[j]));
+  }
+#pragma unroll
+  for (int j = 0; j < 4; j++)
+#pragma unroll
+    for (int h = 0; h < 2; h++)
+#pragma unroll
+      for (int i = 0; i < 4; i++) {
+        const int r = r0 + wm * 32 + i * 8 + fr, c = c0 + wn * 32 + j * 8 + 2 * fk + h;
+        if (r < M && c < M) {
+          double* p = g + r + (i64)c * M;
+          *p = *p + acc[i][j][h];
+        }
+      }
+}
+
+cudaError_t launch_pivchol(const i64* dims, const i64* steps_box, double* G, double* Rws, const i64* qoff, int* perm,
+                           const i64* xoff, double* state, int maxsteps, int nboxes, int maxM, cudaStream_t st) {
   if (nboxes == 0) return cudaSuccess;
-  size_t smem = sizeof(double) * (size_t)maxM + 16;
-  note_launch();
-  k_pivchol_panel<<<nboxes, 256, smem, st>>>(dims, steps_box, G, Rws, qoff, perm, xoff, state, k0, nb);
-  return cudaGetLastError();
+  if (maxM > 8 * PC_NT) return cudaErrorInvalidValue;
+  const size_t smem = sizeof(double) * (size_t)PC_NB * maxM;
+  const bool sm = smem <= 200 * 1024;
+  auto go = [&](auto kern, int k0) {
+    if (sm) {
+      const cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+      if (e != cudaSuccess) return e;
+    }
+    note_launch();
+    kern<<<nboxes, PC_NT, sm ? smem : 0, st>>>(dims, steps_box, G, Rws, qoff, perm, xoff, state, k0);
+    return cudaGetLastError();
+  };
+  const int nt = (maxM + PC_T - 1) / PC_T;
+  for (int k0 = 0; k0 < maxsteps; k0 += PC_NB) {
+    const cudaError_t e = maxM <= PC_NT       ? go(k_pivchol_panel<1, true>, k0)
+                          : maxM <= 2 * PC_NT ? go(k_pivchol_panel<2, true>, k0)
+                          : sm                ? go(k_pivchol_panel<4, true>, k0)
+                                              : go(k_pivchol_panel<8, false>, k0);
+    if (e != cudaSuccess) return e;
+    if (k0 + PC_NB >= maxsteps) break;
+    note_launch();
+    k_pivchol_update<<<dim3(nboxes, nt * nt), 128, 0, st>>>(dims, steps_box, G, Rws, qoff, k0);
+    const cudaError_t e2 = cudaGetLastError();
+    if (e2 != cudaSuccess) return e2;
+  }
+  return cudaSuccess;
 }
 
 }  // namespace h2b

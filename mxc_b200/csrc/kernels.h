@@ -87,11 +87,10 @@ cudaError_t launch_qr_extract(const QrExtractTask<T>* d_tasks, int ntasks, cudaS
 template <typename T>
 cudaError_t launch_wy_t(const WyTask<T>* d_tasks, int ntasks, int maxr, cudaStream_t st);
 
-// Blocked pivoted Cholesky: one panel of nb pivots starting at k0 for every
-// box (steps_box[i] pivots in all); state holds 3 doubles per box.
-cudaError_t launch_pivchol_panel(const i64* dims, const i64* steps_box, double* G, double* Rws, const i64* qoff,
-                                 int* perm, const i64* xoff, double* state, int k0, int nb, int nboxes, int maxM,
-                                 cudaStream_t st);
+// Blocked pivoted Cholesky of every box's Gram matrix (steps_box[i] pivots,
+// maxsteps the largest); state: 3 doubles per box of scratch.
+cudaError_t launch_pivchol(const i64* dims, const i64* steps_box, double* G, double* Rws, const i64* qoff, int* perm,
+                           const i64* xoff, double* state, int maxsteps, int nboxes, int maxM, cudaStream_t st);
 cudaError_t launch_gather_points(const double* bodies, const int* idx, i64 n, double* out, cudaStream_t st);
 // Gram matrix G = X^T X of one box (k_gram): X is S x M column-major.
 struct GramTask {

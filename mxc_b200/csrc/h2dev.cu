@@ -1566,9 +1566,6 @@ class Solver : public SolverBase {
     Rws.alloc(lv.qoff[nodes]);
     Rws.zero(st());
     {
-      // Blocked pivoted Cholesky: panels of 32 pivots per box, each followed
-      // by one batched rank-32 update of every trailing Gram matrix.
-      const int nb = 32;
       std::vector<i64> steps(nodes, 0);
       i64 maxsteps = 0;
       double fl = 0.;
@@ -1623,14 +1620,12 @@ class Solver : public SolverBase {
   // Orthogonal completion (h2matrix.cpp:43-49) for every box with
   // 0 < rank < M, after the finish kernel left U_ID = P [I; T^T] in R's slot
   // and Q_in (upper triangular) in Q: W = Q_in U_ID (M x rank, ld M), a
-  // blocked Householder QR of W (panels factored in shared memory, the
-  // trailing columns updated by three batched GEMMs per panel,
-  // A -= V (T^T (V^T A))), R = triu(W[:rank, :rank]) and
+  // blocked Householder QR of W, R = triu(W[:rank, :rank]) and
   // Q = H_0 ... H_{rank-1} in compact-WY form.
   template <typename U>
   void blocked_orth_qr(Level<T>& lv, U* W, U* Q, U* R, U* taus, const std::vector<i64>& ranks, bool leaf) {
     std::vector<i64> box;
-    i64 maxM = 0, maxr = 0, ysz = 0;
+    i64 maxM = 0, maxr = 0;
     for (i64 i = 0; i < lv.nodes; i++) {
       const i64 M = lv.dims[i], r = ranks[i];
       if (!(0 < r && r < M)) continue;
@@ -1639,9 +1634,7 @@ class Solver : public SolverBase {
       maxr = std::max(maxr, r);
     }
     if (box.empty()) return;
-    int nb = 32;
-    while (nb > 1 && sizeof(U) * ((size_t)maxM * nb + 2 * nb + (size_t)nb * nb) > 190 * 1024) nb--;
-    for (i64 i : box) ysz += (i64)nb * ranks[i];
+    const i64 nb = qr_panel_width((int)maxM, sizeof(U));
     {
       double fl = 0.;
       for (i64 i : box) fl += leaf ? 0. : (double)lv.dims[i] * lv.dims[i] * ranks[i];
@@ -1662,60 +1655,28 @@ class Solver : public SolverBase {
         g.run(st());
       }
     }
-    DVec<U> Vp, Tp, Y, Y2;
+    DVec<U> Vp, Tp;
     Vp.alloc((i64)box.size() * maxM * nb);
     Tp.alloc((i64)box.size() * nb * nb);
-    Y.alloc(ysz);
-    Y2.alloc(ysz);
-    for (i64 k0 = 0; k0 < maxr; k0 += nb) {
+    {
       std::vector<QrPanelTask<U>> pt;
-      GemmPlan<U> gy, gt, ga;
-      gy.name = gt.name = ga.name = "gemm_qr";
-      i64 yo = 0;
-      int maxm = 0;
       double fl = 0.;
       for (size_t z = 0; z < box.size(); z++) {
         const i64 i = box[z], M = lv.dims[i], r = ranks[i];
-        if (k0 >= r) continue;
-        const int w = (int)std::min<i64>(nb, r - k0), m = (int)(M - k0);
-        U* vp = Vp.p + (i64)z * maxM * nb;
-        U* tp = Tp.p + (i64)z * nb * nb;
         QrPanelTask<U> t;
         t.W = W + lv.qoff[i];
-        t.Vp = vp;
-        t.Tp = tp;
+        t.Vp = Vp.p + (i64)z * maxM * nb;
+        t.Tp = Tp.p + (i64)z * nb * nb;
         t.taus = taus + lv.xoff[i];
         t.M = (int)M;
-        t.k0 = (int)k0;
-        t.nb = w;
+        t.rank = (int)r;
         pt.push_back(t);
-        maxm = std::max(maxm, m);
-        fl += 2. * m * w * w;
-        const i64 n2 = r - k0 - w;
-        if (n2 <= 0) continue;
-        U* At = W + lv.qoff[i] + k0 + (k0 + w) * M;
-        gy.add_task(Y.p + yo, w, w, (int)n2, U(0));
-        gy.add_entry(vp, m, 1, At, M, 0, m, U(1));
-        gt.add_task(Y2.p + yo, w, w, (int)n2, U(0));
-        gt.add_entry(tp, w, 1, Y.p + yo, w, 0, w, U(1));
-        ga.add_task(At, M, m, (int)n2, U(1));
-        ga.add_entry(vp, m, 0, Y2.p + yo, w, 0, w, U(-1));
-        yo += (i64)w * n2;
+        fl += 2. * M * r * r;
       }
       DVec<QrPanelTask<U>> dpt;
       dpt.upload(pt);
-      {
-        Prof pf("qr_panel", fl, 0.);
-        ck(launch_qr_panel<U>(dpt.p, (int)pt.size(), maxm, nb, st()), "qr_panel");
-      }
-      if (yo > 0) {
-        gy.finalize();
-        gt.finalize();
-        ga.finalize();
-        gy.run(st());
-        gt.run(st());
-        ga.run(st());
-      }
+      Prof pf("blocked_qr", fl, 0.);
+      ck(launch_blocked_qr<U>(dpt.p, (int)pt.size(), (int)maxM, (int)maxr, st()), "blocked_qr");
     }
     std::vector<QrExtractTask<U>> et;
     for (i64 i : box) {

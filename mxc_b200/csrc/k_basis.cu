@@ -901,16 +901,190 @@ template cudaError_t launch_wy_t<float>(const WyTask<float>*, int, int, cudaStre
 namespace h2b {
 
 // One Householder panel of the M x rank matrix W (column-major, ld M) of a
-// box: columns k0..k0+nb-1, rows k0..M-1, factored in shared memory with the
-// same reflector convention as the reference (beta = -sign(c0) * norm).
-// Writes back R (upper) and the reflector tails (lower), the explicit unit
-// lower-trapezoidal V of the panel to Vp ((M-k0) x nb), the panel's
-// compact-WY T (nb x nb, I - V T V^T = H_k0 ... H_k0+nb-1) to Tp and its
-// taus.  The caller applies the panel to the trailing columns with GEMMs.
+// box: columns k0..k0+nb-1, rows k0..M-1, factored with the reference's
+// reflector convention (beta = -sign(c0) * norm).  Writes back R (upper) and
+// the reflector tails (lower), the explicit unit lower-trapezoidal V of the
+// panel to Vp ((M-k0) x nb), the panel's compact-WY T (nb x nb, I - V T V^T =
+// H_k0 ... H_k0+nb-1) to Tp and its taus.  k_qr_update applies the panel to the
+// trailing columns.
+//
+// Bound: the chain of columns.  k_qr_panel keeps the panel in registers (rows
+// over the lanes, RPL per lane; warp w the columns w, w + 8, ...) and needs two
+// barriers per column -- the column published to shared memory, its norm's
+// partial sums -- so a column costs the latency of one norm, one square root,
+// a division and one dot product; with the panel in shared memory and a block
+// reduction per column it was 5 us a column whatever the number of boxes
+// (65,536 bodies, rank 128: panels and updates 6.7 -> 3.5 ms over eight levels).
+// The sums keep their order (row k + 1 + i in lane i mod 32 of the norm and the
+// dot products), hence the rotations.  Taller panels run k_qr_panel_smem.
 template <typename T>
-__global__ void __launch_bounds__(256) k_qr_panel(const QrPanelTask<T>* __restrict__ tasks) {
+__device__ __forceinline__ void qr_panel_finish(const QrPanelTask<T>& t, const T* P, T* Tl, T* sc, const T* tau, int m,
+                                                int nb, int k0) {
+  const int tid = threadIdx.x, nt = blockDim.x, lane = tid & 31, warp = tid >> 5, nw = nt >> 5;
+  T* Wp = t.W + (i64)k0 + (i64)k0 * t.M;
+  // S[l][i] = V(:,l)^T V(:,i) for l < i (V unit lower: V[i][i] = 1, zero above),
+  // four l of one i at a time.
+  for (int e = warp; e < nb * ((nb + 3) / 4); e += nw) {
+    const int i = e % nb, l0 = e / nb * 4;
+    if (l0 >= i) continue;
+    T s[4] = {0, 0, 0, 0};
+    for (int r = i + 1 + lane; r < m; r += 32) {
+      const T x = P[r + (size_t)i * m];
+#pragma unroll
+      for (int u = 0; u < 4; u++)
+        if (l0 + u < i) s[u] += P[r + (size_t)(l0 + u) * m] * x;
+    }
+    for (int o = 16; o > 0; o >>= 1)
+#pragma unroll
+      for (int u = 0; u < 4; u++) s[u] += __shfl_xor_sync(0xffffffffu, s[u], o);
+    if (lane == 0)
+#pragma unroll
+      for (int u = 0; u < 4; u++)
+        if (l0 + u < i) Tl[l0 + u + i * nb] = s[u] + P[i + (size_t)(l0 + u) * m];  // row i of V(:,l) times V[i][i] = 1
+  }
+  __syncthreads();
+  // T recurrence, one warp: column i of S is staged in sc, then
+  // T[:i, i] = -tau_i T[:i,:i] S[:i, i] and T[i][i] = tau_i.
+  if (warp == 0) {
+    for (int i = 0; i < nb; i++) {
+      for (int j = lane; j < i; j += 32) sc[j] = Tl[j + i * nb];
+      __syncwarp();
+      for (int j = lane; j < i; j += 32) {
+        T v = 0;
+        for (int l = j; l < i; l++) v += Tl[j + l * nb] * sc[l];
+        Tl[j + i * nb] = -tau[i] * v;
+      }
+      if (lane == 0) Tl[i + i * nb] = tau[i];
+      __syncwarp();
+    }
+  } else {
+    for (int e = tid - 32, n = nt - 32; e < m * nb; e += n) {
+      const int r = e % m, j = e / m;
+      Wp[r + (i64)j * t.M] = P[e];
+      t.Vp[e] = r < j ? T(0) : (r == j ? T(1) : P[e]);
+    }
+  }
+  __syncthreads();
+  for (int e = tid; e < nb * nb; e += nt) {
+    int r = e % nb, c = e / nb;
+    t.Tp[e] = r <= c ? Tl[e] : T(0);
+  }
+  for (int j = tid; j < nb; j += nt) t.taus[k0 + j] = tau[j];
+}
+
+constexpr int QP_NT = 256, QP_NB = 32;
+
+template <typename T, int RPL>
+__global__ void __launch_bounds__(QP_NT) k_qr_panel(const QrPanelTask<T>* __restrict__ tasks, int k0) {
+  constexpr int NW = QP_NT / 32, CPW = QP_NB / NW;
   const QrPanelTask<T> t = tasks[blockIdx.x];
-  const int m = t.M - t.k0, nb = t.nb;
+  if (k0 >= t.rank) return;
+  const int m = t.M - k0, nb = min(QP_NB, t.rank - k0);
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  T* P = reinterpret_cast<T*>(smem_raw);  // m x nb, ld m
+  T* Tl = P + (size_t)m * nb;             // nb x nb
+  __shared__ T col[2][RPL * 32];          // published column
+  __shared__ T tau[QP_NB], sc[QP_NB], red[2][NW];
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const T* Wp = t.W + (i64)k0 + (i64)k0 * t.M;
+  T x[CPW][RPL];
+#pragma unroll
+  for (int u = 0; u < CPW; u++)
+#pragma unroll
+    for (int i = 0; i < RPL; i++) {
+      const int r = lane + 32 * i, c = warp + NW * u;
+      x[u][i] = (r < m && c < nb) ? Wp[r + (i64)c * t.M] : T(0);
+    }
+  for (int j = 0; j < nb; j++) {
+    const int ow = j % NW, os = j / NW, b = j & 1;
+    if (warp == ow) {
+#pragma unroll
+      for (int u = 0; u < CPW; u++)
+        if (u == os)
+#pragma unroll
+          for (int i = 0; i < RPL; i++) col[b][lane + 32 * i] = x[u][i];
+    }
+    __syncthreads();
+    // Norm below the diagonal, in the order of a block reduction over rows.
+    T part = 0;
+    for (int r = j + 1 + tid; r < m; r += QP_NT) part += col[b][r] * col[b][r];
+    for (int o = 16; o > 0; o >>= 1) part += __shfl_xor_sync(0xffffffffu, part, o);
+    if (lane == 0) red[b][warp] = part;
+    T v[RPL];
+#pragma unroll
+    for (int i = 0; i < RPL; i++) v[i] = col[b][lane + 32 * i];
+    const T c0 = col[b][j];
+    __syncthreads();
+    const T* rb = red[b];
+    const T tsq = ((rb[0] + rb[4]) + (rb[2] + rb[6])) + ((rb[1] + rb[5]) + (rb[3] + rb[7]));
+    T tj = 0, beta = c0, scale = 0;
+    if (tsq > Tiny<T>::v()) {
+      beta = sqrt(c0 * c0 + tsq);
+      if (c0 >= T(0)) beta = -beta;
+      scale = T(1) / (c0 - beta);
+      tj = (beta - c0) / beta;
+    }
+#pragma unroll
+    for (int i = 0; i < RPL; i++) {
+      const int r = lane + 32 * i;
+      v[i] = (r > j && r < m) ? v[i] * scale : T(0);
+    }
+    if (warp == ow) {
+#pragma unroll
+      for (int u = 0; u < CPW; u++)
+        if (u == os)
+#pragma unroll
+          for (int i = 0; i < RPL; i++) {
+            const int r = lane + 32 * i;
+            if (r > j) x[u][i] = v[i];
+            if (r == j) x[u][i] = beta;
+          }
+      if (lane == 0) tau[j] = tj;
+    }
+    if (tj != T(0) && warp + NW * (CPW - 1) > j) {  // else none of this warp's columns is left
+      T w[CPW], cj[CPW];
+#pragma unroll
+      for (int u = 0; u < CPW; u++) {
+        T s = 0;
+#pragma unroll
+        for (int i = 0; i < RPL; i++) s += v[i] * x[u][i];
+        cj[u] = __shfl_sync(0xffffffffu, x[u][0], j);  // row j (j < 32)
+        w[u] = __shfl_sync(0xffffffffu, s, (lane + j + 1) & 31);
+      }
+      for (int o = 16; o > 0; o >>= 1)
+#pragma unroll
+        for (int u = 0; u < CPW; u++) w[u] += __shfl_xor_sync(0xffffffffu, w[u], o);
+#pragma unroll
+      for (int u = 0; u < CPW; u++) {
+        if (warp + NW * u <= j) continue;
+        const T wu = (w[u] + cj[u]) * tj;
+#pragma unroll
+        for (int i = 0; i < RPL; i++) {
+          const int r = lane + 32 * i;
+          if (r > j)
+            x[u][i] -= wu * v[i];
+          else if (r == j)
+            x[u][i] -= wu;
+        }
+      }
+    }
+  }
+#pragma unroll
+  for (int u = 0; u < CPW; u++)
+#pragma unroll
+    for (int i = 0; i < RPL; i++) {
+      const int r = lane + 32 * i, c = warp + NW * u;
+      if (r < m && c < nb) P[r + (size_t)c * m] = x[u][i];
+    }
+  __syncthreads();
+  qr_panel_finish(t, P, Tl, sc, tau, m, nb, k0);
+}
+
+template <typename T>
+__global__ void __launch_bounds__(256) k_qr_panel_smem(const QrPanelTask<T>* __restrict__ tasks, int k0, int nbmax) {
+  const QrPanelTask<T> t = tasks[blockIdx.x];
+  if (k0 >= t.rank) return;
+  const int m = t.M - k0, nb = min(nbmax, t.rank - k0);
   extern __shared__ __align__(16) unsigned char smem_raw[];
   T* P = reinterpret_cast<T*>(smem_raw);  // m x nb, ld m
   T* tau = P + (size_t)m * nb;            // nb
@@ -918,7 +1092,7 @@ __global__ void __launch_bounds__(256) k_qr_panel(const QrPanelTask<T>* __restri
   T* sc = Tl + (size_t)nb * nb;           // nb
   __shared__ T red[32];
   const int tid = threadIdx.x, nt = blockDim.x, lane = tid & 31, warp = tid >> 5, nw = nt >> 5;
-  T* Wp = t.W + (i64)t.k0 + (i64)t.k0 * t.M;
+  const T* Wp = t.W + (i64)k0 + (i64)k0 * t.M;
   for_each_rc(m, nb, [&](int r, int j, int e) {
     P[e] = Wp[r + (i64)j * t.M];
   });
@@ -955,56 +1129,170 @@ __global__ void __launch_bounds__(256) k_qr_panel(const QrPanelTask<T>* __restri
       }
     __syncthreads();
   }
-  // S[l][i] = V(:,l)^T V(:,i) for l < i (V unit lower: V[i][i] = 1, zero above).
-  for (int pr = warp; pr < nb * nb; pr += nw) {
-    int l = pr % nb, i = pr / nb;
-    if (l >= i) continue;
-    T s = 0;
-    for (int r = i + 1 + lane; r < m; r += 32) s += P[r + (size_t)l * m] * P[r + (size_t)i * m];
-    for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
-    if (lane == 0) Tl[l + i * nb] = s + P[i + (size_t)l * m];  // row i of V(:,l) times V[i][i] = 1
+  qr_panel_finish(t, P, Tl, sc, tau, m, nb, k0);
+}
+
+// The panel applied to the trailing columns, A -= V (T^T (V^T A)): one CTA per
+// box and QU_C columns of A (rows k0..M-1).  The three products run in one
+// launch (three GEMM launches and their host-built task lists a panel before):
+// FP64 on the tensor cores (mma.sync m8n8k4, V and A read where they lie, their
+// four consecutive k of a fragment being one 32-byte sector), FP32 on the FMA
+// pipe (bases of the Householder mode only).
+constexpr int QU_C = 32;
+
+template <typename T>
+__global__ void __launch_bounds__(256) k_qr_update(const QrPanelTask<T>* __restrict__ tasks, int k0, int nbmax) {
+  constexpr int LD = 36;
+  const QrPanelTask<T> t = tasks[blockIdx.x];
+  const int nb = min(nbmax, t.rank - k0), m = t.M - k0;
+  const int c0 = k0 + nb + blockIdx.y * QU_C;
+  if (nb <= 0 || c0 >= t.rank) return;
+  const int nc = min(QU_C, t.rank - c0);
+  __shared__ T Y[QU_C][LD], Y2[QU_C][LD], Ts[QU_C][LD];  // [column][row]
+  const T* V = t.Vp;  // m x nb, ld m
+  T* A = t.W + k0 + (i64)c0 * t.M;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  for (int e = tid; e < 32 * 32; e += 256) {
+    const int r = e & 31, c = e >> 5;
+    Ts[c][r] = (r < nb && c < nb) ? t.Tp[r + c * nb] : T(0);
   }
-  __syncthreads();
-  // T recurrence, one warp: column i of S is staged in sc, then
-  // T[:i, i] = -tau_i T[:i,:i] S[:i, i] and T[i][i] = tau_i.
-  if (warp == 0) {
-    for (int i = 0; i < nb; i++) {
-      for (int j = lane; j < i; j += 32) sc[j] = Tl[j + i * nb];
-      __syncwarp();
-      for (int j = lane; j < i; j += 32) {
-        T v = 0;
-        for (int l = j; l < i; l++) v += Tl[j + l * nb] * sc[l];
-        Tl[j + i * nb] = -tau[i] * v;
+  if constexpr (sizeof(T) == 8) {
+    const int fr = lane >> 2, fk = lane & 3;
+    auto mma = [](double (&d)[2], double a, double b) {
+      asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0, %1}, {%2}, {%3}, {%0, %1};\n"
+                   : "+d"(d[0]), "+d"(d[1])
+                   : "d"(a), "d"(b));
+    };
+    // Y = V^T A: warp w has rows 8 (w % 4).. and the two column groups w / 4, + 2.
+    const int yr = 8 * (warp & 3) + fr, yc = 8 * (warp >> 2) + fr;
+    double y[2][2] = {{0., 0.}, {0., 0.}};
+    const bool av = yr < nb, bv0 = yc < nc, bv1 = yc + 16 < nc;
+    const double *va = V + (i64)yr * m + fk, *a0 = A + (i64)yc * t.M + fk, *a1 = a0 + 16 * (i64)t.M;
+    for (int k = 0; k < m; k += 32) {
+      double fa[8], f0[8], f1[8];
+#pragma unroll
+      for (int i = 0; i < 8; i++) {
+        const bool kv = k + 4 * i + fk < m;
+        fa[i] = (av && kv) ? va[k + 4 * i] : 0.;
+        f0[i] = (bv0 && kv) ? a0[k + 4 * i] : 0.;
+        f1[i] = (bv1 && kv) ? a1[k + 4 * i] : 0.;
       }
-      if (lane == 0) Tl[i + i * nb] = tau[i];
-      __syncwarp();
+#pragma unroll
+      for (int i = 0; i < 8; i++) {
+        mma(y[0], fa[i], f0[i]);
+        mma(y[1], fa[i], f1[i]);
+      }
     }
+#pragma unroll
+    for (int i = 0; i < 2; i++)
+#pragma unroll
+      for (int h = 0; h < 2; h++) Y[8 * (warp >> 2) + 16 * i + 2 * fk + h][yr] = y[i][h];
+    __syncthreads();
+    // Y2 = T^T Y (T[k][row] at Ts[row][k]).
+    y[0][0] = y[0][1] = y[1][0] = y[1][1] = 0.;
+#pragma unroll
+    for (int k = 0; k < 32; k += 4)
+#pragma unroll
+      for (int i = 0; i < 2; i++) mma(y[i], Ts[yr][k + fk], Y[yc + 16 * i][k + fk]);
+#pragma unroll
+    for (int i = 0; i < 2; i++)
+#pragma unroll
+      for (int h = 0; h < 2; h++) Y2[8 * (warp >> 2) + 16 * i + 2 * fk + h][yr] = y[i][h];
+    __syncthreads();
+    // A -= V Y2, 16 rows x 32 columns a warp at a time.
+    for (int r0 = 16 * warp; r0 < m; r0 += 128) {
+      double acc[2][4][2];
+#pragma unroll
+      for (int i = 0; i < 2; i++)
+#pragma unroll
+        for (int j = 0; j < 4; j++) acc[i][j][0] = acc[i][j][1] = 0.;
+      double fa[2][8];
+#pragma unroll
+      for (int i = 0; i < 2; i++)
+#pragma unroll
+        for (int k = 0; k < 8; k++) {
+          const int r = r0 + 8 * i + fr, kk = 4 * k + fk;
+          fa[i][k] = (r < m && kk < nb) ? -V[r + (i64)kk * m] : 0.;
+        }
+#pragma unroll
+      for (int k = 0; k < 8; k++)
+#pragma unroll
+        for (int j = 0; j < 4; j++) {
+          const double f = Y2[8 * j + fr][4 * k + fk];
+          mma(acc[0][j], fa[0][k], f);
+          mma(acc[1][j], fa[1][k], f);
+        }
+#pragma unroll
+      for (int j = 0; j < 4; j++)
+#pragma unroll
+        for (int h = 0; h < 2; h++)
+#pragma unroll
+          for (int i = 0; i < 2; i++) {
+            const int r = r0 + 8 * i + fr, c = 8 * j + 2 * fk + h;
+            if (r < m && c < nc) {
+              double* p = A + r + (i64)c * t.M;
+              *p = *p + acc[i][j][h];
+            }
+          }
+    }
+  } else {
+    for (int e = tid; e < 32 * 32; e += 256) {
+      const int r = e & 31, c = e >> 5;
+      T s = T(0);
+      if (r < nb && c < nc)
+        for (int k = 0; k < m; k++) s += V[k + (i64)r * m] * A[k + (i64)c * t.M];
+      Y[c][r] = s;
+    }
+    __syncthreads();
+    for (int e = tid; e < 32 * 32; e += 256) {
+      const int r = e & 31, c = e >> 5;
+      T s = T(0);
+      for (int k = 0; k <= r; k++) s += Ts[r][k] * Y[c][k];
+      Y2[c][r] = s;
+    }
+    __syncthreads();
+    for_each_rc(m, nc, [&](int r, int c, int) {
+      T s = T(0);
+      for (int k = 0; k < nb; k++) s += V[r + (i64)k * m] * Y2[c][k];
+      A[r + (i64)c * t.M] -= s;
+    });
   }
-  __syncthreads();
-  for_each_rc(m, nb, [&](int r, int j, int e) {
-    Wp[r + (i64)j * t.M] = P[e];
-    t.Vp[e] = r < j ? T(0) : (r == j ? T(1) : P[e]);
-  });
-  for (int e = tid; e < nb * nb; e += nt) {
-    int r = e % nb, c = e / nb;
-    t.Tp[e] = r <= c ? Tl[e] : T(0);
-  }
-  for (int j = tid; j < nb; j += nt) t.taus[t.k0 + j] = tau[j];
+}
+
+int qr_panel_width(int maxM, size_t elem) {
+  if (maxM <= 512) return QP_NB;
+  int nb = QP_NB;
+  while (nb > 1 && elem * ((size_t)maxM * nb + 2 * nb + (size_t)nb * nb) > 190 * 1024) nb--;
+  return nb;
 }
 
 template <typename T>
-cudaError_t launch_qr_panel(const QrPanelTask<T>* d_tasks, int ntasks, int maxm, int nb, cudaStream_t st) {
+cudaError_t launch_blocked_qr(const QrPanelTask<T>* d_tasks, int ntasks, int maxM, int maxr, cudaStream_t st) {
   if (ntasks == 0) return cudaSuccess;
-  size_t smem = sizeof(T) * ((size_t)maxm * nb + 2 * nb + (size_t)nb * nb) + 16;
-  auto fn = k_qr_panel<T>;
-  cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-  if (e != cudaSuccess) return e;
-  note_launch();
-  fn<<<ntasks, 256, smem, st>>>(d_tasks);
-  return cudaGetLastError();
+  const int nb = qr_panel_width(maxM, sizeof(T));
+  for (int k0 = 0; k0 < maxr; k0 += nb) {
+    const int m = maxM - k0;
+    auto go = [&](auto kern, auto... more) {
+      const size_t smem = sizeof(T) * ((size_t)m * nb + 2 * nb + (size_t)nb * nb) + 16;
+      const cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+      if (e != cudaSuccess) return e;
+      note_launch();
+      kern<<<ntasks, 256, smem, st>>>(d_tasks, k0, more...);
+      return cudaGetLastError();
+    };
+    // 256 rows: 8 a lane; up to 512: 16.
+    cudaError_t e = maxM > 512 ? go(k_qr_panel_smem<T>, nb) : m <= 256 ? go(k_qr_panel<T, 8>) : go(k_qr_panel<T, 16>);
+    if (e != cudaSuccess) return e;
+    if (k0 + nb >= maxr) break;
+    note_launch();
+    k_qr_update<T><<<dim3(ntasks, (maxr - k0 - nb + QU_C - 1) / QU_C), 256, 0, st>>>(d_tasks, k0, nb);
+    e = cudaGetLastError();
+    if (e != cudaSuccess) return e;
+  }
+  return cudaSuccess;
 }
-template cudaError_t launch_qr_panel<double>(const QrPanelTask<double>*, int, int, int, cudaStream_t);
-template cudaError_t launch_qr_panel<float>(const QrPanelTask<float>*, int, int, int, cudaStream_t);
+template cudaError_t launch_blocked_qr<double>(const QrPanelTask<double>*, int, int, int, cudaStream_t);
+template cudaError_t launch_blocked_qr<float>(const QrPanelTask<float>*, int, int, int, cudaStream_t);
 
 }  // namespace h2b
 

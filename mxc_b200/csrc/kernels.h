@@ -64,17 +64,18 @@ struct WyTask {
   T* Tm;          // r x r output (upper triangular)
   int r;
 };
-// One Householder panel per box (k_qr_panel).
+// Blocked Householder QR of every box's W (M x rank, column-major, ld M).
 template <typename T>
 struct QrPanelTask {
-  T* W;      // M x rank, column-major (ld M)
-  T* Vp;     // (M - k0) x nb explicit V of the panel
-  T* Tp;     // nb x nb
-  T* taus;   // per box, indexed by column
-  int M, k0, nb;
+  T* W;
+  T* Vp;    // scratch: M x qr_panel_width, the panel's explicit V
+  T* Tp;    // scratch: qr_panel_width^2, its T
+  T* taus;  // indexed by column
+  int M, rank;
 };
+int qr_panel_width(int maxM, size_t elem);
 template <typename T>
-cudaError_t launch_qr_panel(const QrPanelTask<T>* d_tasks, int ntasks, int maxm, int nb, cudaStream_t st);
+cudaError_t launch_blocked_qr(const QrPanelTask<T>* d_tasks, int ntasks, int maxM, int maxr, cudaStream_t st);
 template <typename T>
 struct QrExtractTask {
   T* W;

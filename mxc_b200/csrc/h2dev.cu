@@ -385,6 +385,26 @@ static int tuned_variant(const std::string& key, int nvar, cudaStream_t st, F ru
   return rec.choice;
 }
 
+// Whether a streaming plan runs by rows (k_apply): with at most 4 right-hand
+// sides always (near field of 20,000 bodies, 1 column: 186 -> 150 us; a level's
+// small pass 15 -> 8.5), with more only where the latency of a launch counts --
+// few row tiles and short sums (16 columns, K 256: 128 boxes 27 -> 25 us, 16
+// boxes 17 -> 12.5, but 512 boxes 52 -> 72; sums over 27 neighbours, K 3456:
+// 128 boxes 76 -> 109 us), where the ring's split tasks need a second launch.
+template <typename TK, typename EN>
+static bool apply_by_rows(int nr, const std::vector<TK>& tasks, const std::vector<EN>& ents) {
+  if (nr <= 4) return true;
+  double rowtiles = 0.;
+  i64 longest = 0;
+  for (const auto& t : tasks) {
+    rowtiles += (t.m + 127) / 128;
+    i64 k = 0;
+    for (int e = t.e0; e < t.e1; e++) k += ents[e].k;
+    longest = std::max(longest, k);
+  }
+  return rowtiles <= 256. && longest <= 512;
+}
+
 // Host-built list of segmented-GEMM tasks, uploaded once and replayed.
 template <typename T>
 struct GemmPlan {
@@ -410,6 +430,9 @@ struct GemmPlan {
   // Only plans that overwrite their outputs (every beta zero) are timed:
   // repeating one leaves the same result, so tuning runs are harmless.
   bool idempotent = false;
+  // By-rows plans (k_apply): d_rtiles / d_rtiles_w are the tilings of 1 and 2
+  // rows per lane, the autotuner's two variants.
+  bool by_rows = false;
   // FP64 streaming plans whose A columns all start on 16-byte boundaries run
   // the bulk-copy kernel.
   bool bulk_ok = false;
@@ -446,8 +469,27 @@ struct GemmPlan {
     // its ordered sum and gives the parts beta zero.
     idempotent = true;
     for (const auto& t : tasks) idempotent = idempotent && t.beta == T(0);
-    if (skinny_nn) split_tasks();
     if (skinny_nn) {
+      by_rows = apply_by_rows(nr, tasks, ents);
+    }
+    if (skinny_nn && by_rows) {
+      std::vector<int2> rt[2];
+      double rows = 0., elems = 0.;
+      for (int ti = 0; ti < (int)tasks.size(); ti++) {
+        const auto& t = tasks[ti];
+        if (t.m <= 0 || t.n <= 0) continue;
+        if (t.e0 == t.e1 && t.beta == T(1)) continue;
+        for (int v = 0; v < 2; v++)
+          for (int a = 0; a < t.m; a += apply_rows_per_cta(v + 1)) rt[v].push_back(make_int2(ti, a / apply_rows_per_cta(v + 1)));
+        rows += t.m;
+        for (int e = t.e0; e < t.e1; e++) elems += (double)t.m * ents[e].k;
+      }
+      d_rtiles.upload(rt[0]);
+      d_rtiles_w.upload(rt[1]);
+      tkey = tune_key(name, (int)sizeof(T), nr, (double)tasks.size(), rows, elems);
+    }
+    if (skinny_nn && !by_rows) split_tasks();
+    if (skinny_nn && !by_rows) {
       // A task takes 256-row tiles when they leave no more padding rows
       // than 128-row tiles would, else 128-row tiles (two launches back to
       // back; padding rows are zero-filled copies whose tensor-core work is
@@ -616,6 +658,11 @@ struct GemmPlan {
   }
 
   void run_skinny(int v, cudaStream_t st) const {
+    if (by_rows) {
+      const DVec<int2>& t = v == 0 ? d_rtiles_w : d_rtiles;
+      ck(launch_apply<T>(nr, v == 0 ? 2 : 1, d_tasks.p, d_ents.p, t.p, (int)t.n, st), "apply");
+      return;
+    }
     const DVec<int2>& w = v == 0 ? d_rtiles_w : d_alt_w;
     const DVec<int2>& n = v == 0 ? d_rtiles : d_alt_n;
     int* be = (bulk_ok && g_cur) ? g_cur->d_tc_err : nullptr;
@@ -632,7 +679,7 @@ struct GemmPlan {
       variant = 0;
       return;
     }
-    const int v = tuned_variant(tkey, 3, st, [&](int x) { run_skinny(x, st); });
+    const int v = tuned_variant(tkey, by_rows ? 2 : 3, st, [&](int x) { run_skinny(x, st); });
     if (!stream_capturing(st)) variant = v;
   }
 
@@ -749,9 +796,11 @@ struct BfPlan {
   DVec<float> parts_buf;
   DVec<SumTask<float>> d_sums;
   int nsums = 0, sum_maxmn = 0;
+  bool by_rows = false;  // as GemmPlan::by_rows (2 rows per lane)
   void finalize() {
-    split();
-    const int bm = bf16_rows_per_cta();
+    by_rows = apply_by_rows(nr, tasks, ents);
+    if (!by_rows) split();
+    const int bm = by_rows ? apply_rows_per_cta(2) : bf16_rows_per_cta();
     tiles.clear();
     for (size_t t = 0; t < tasks.size(); t++)
       for (int r = 0; r < tasks[t].m; r += bm) tiles.push_back(make_int2((int)t, r / bm));
@@ -848,6 +897,10 @@ struct BfPlan {
   }
   void run(cudaStream_t st) const {
     Prof p("bf16_precond", flops, bytes, st);
+    if (by_rows) {
+      ck(launch_apply_bf16(nr, 2, d_tasks.p, d_ents.p, d_tiles.p, (int)tiles.size(), st), "apply_bf16");
+      return;
+    }
     ck(launch_stream_bf16(nr, d_tasks.p, d_ents.p, d_tiles.p, (int)tiles.size(), st), "bf16_precond");
     if (nsums) ck(launch_sum_parts<float>(d_sums.p, nsums, sum_maxmn, st), "sum_parts");
   }
@@ -1005,7 +1058,7 @@ class Solver : public SolverBase {
   DVec<__nv_bfloat16> bf_pool;
   DVec<float> bf_scales;
   std::vector<BfPlan> bf_fx, bf_fz, bf_bx, bf_by;
-  std::vector<CopyPlan<T>> pc_fcopy, pc_bcopy;
+  std::vector<CopyPlan<T>> pc_fcopy;
   bool mv_built = false, pc_built = false;
 
   cudaStream_t st() const { return h->stream; }
@@ -2247,9 +2300,9 @@ class Solver : public SolverBase {
   void build_precondition(i64 nrhs) {
     const int nr = (int)nrhs;
     gen++;
-    pc_fx.clear(); pc_fz.clear(); pc_bx.clear(); pc_by.clear(); pc_fcopy.clear(); pc_bcopy.clear();
+    pc_fx.clear(); pc_fz.clear(); pc_bx.clear(); pc_by.clear(); pc_fcopy.clear();
     pc_fx.resize(levels + 1); pc_fz.resize(levels + 1); pc_bx.resize(levels + 1); pc_by.resize(levels + 1);
-    pc_fcopy.resize(levels + 1); pc_bcopy.resize(levels + 1);
+    pc_fcopy.resize(levels + 1);
     {
       CopyPlan<T> tp;
       for (i64 l = 0; l <= levels; l++) {
@@ -2272,11 +2325,22 @@ class Solver : public SolverBase {
       for (i64 i = 0; i < lv.nodes; i++) {
         const int M = (int)lv.dims[i], Ms = (int)lv.ranks[i], Mr = M - Ms;
         if (M == 0) continue;
-        // forward: X = V Y; Z = X_s - sum_j A_ij[:Ms, Ns:] X_j[Ns:]
-        pc_fx[l].add_task(X + lv.xoff[i], ldx, M, nr, T(0));
-        pc_fx[l].add_entry(lv.Rt.p + lv.qoff[i], M, 0, Yin + lv.xoff[i], ldx, 0, M, T(1));
+        // forward: [Z; X_r] = V Y, Z -= sum_j A_ij[:Ms, Ns:] X_j[Ns:].  The two
+        // row ranges are tasks of their own, so that the skeleton rows land in
+        // Z; where the second would start off a 16-byte boundary (the ring's
+        // copies) all rows go to X and the skeleton rows are copied.
+        const bool cut = Ms > 0 && (Mr == 0 || Ms * sizeof(T) % 16 == 0);
+        if (cut) {
+          pc_fx[l].add_task(Z + lv.zoff[i], ldz, Ms, nr, T(0));
+          pc_fx[l].add_entry(lv.Rt.p + lv.qoff[i], M, 0, Yin + lv.xoff[i], ldx, 0, M, T(1));
+        }
+        if (!cut || Mr > 0) {
+          const int r0 = cut ? Ms : 0;
+          pc_fx[l].add_task(X + lv.xoff[i] + r0, ldx, M - r0, nr, T(0));
+          pc_fx[l].add_entry(lv.Rt.p + lv.qoff[i] + r0, M, 0, Yin + lv.xoff[i], ldx, 0, M, T(1));
+        }
         if (Ms > 0) {
-          pc_fcopy[l].add(X + lv.xoff[i], ldx, Z + lv.zoff[i], ldz, Ms, nr);
+          if (!cut) pc_fcopy[l].add(X + lv.xoff[i], ldx, Z + lv.zoff[i], ldz, Ms, nr);
           pc_fz[l].add_task(Z + lv.zoff[i], ldz, Ms, nr, T(1));
           for (i64 k = lv.arow[i]; k < lv.arow[i + 1]; k++) {
             i64 j = lv.acol[k];
@@ -2285,8 +2349,7 @@ class Solver : public SolverBase {
               pc_fz[l].add_entry(lv.A.p + lv.aoff[k] + (i64)Ns * M, M, 0, X + lv.xoff[j] + Ns, ldx, 0, Nr, T(-1));
           }
         }
-        // backward: X_s = W; X_r -= sum_j A_ij[Ms:, :Ns] W_j; Y = U X
-        if (Ms > 0) pc_bcopy[l].add(W + lv.zoff[i], ldz, X + lv.xoff[i], ldx, Ms, nr);
+        // backward: X_r -= sum_j A_ij[Ms:, :Ns] W_j; Y = U [W; X_r]
         if (Mr > 0) {
           pc_bx[l].add_task(X + lv.xoff[i] + Ms, ldx, Mr, nr, T(1));
           for (i64 k = lv.arow[i]; k < lv.arow[i + 1]; k++) {
@@ -2297,16 +2360,14 @@ class Solver : public SolverBase {
         }
         const i64 ldy = (l == levels) ? N : L[l + 1].lenZ;
         pc_by[l].add_task(Yout + lv.xoff[i], ldy, M, nr, T(0));
-        pc_by[l].add_entry(lv.Q.p + lv.qoff[i], M, 0, X + lv.xoff[i], ldx, 0, M, T(1));
+        pc_by[l].add_entry(lv.Q.p + lv.qoff[i], M, 0, W + lv.zoff[i], ldz, 0, Ms, T(1));
+        pc_by[l].add_entry(lv.Q.p + lv.qoff[i] + (i64)Ms * M, M, 0, X + lv.xoff[i] + Ms, ldx, 0, Mr, T(1));
       }
       pc_fx[l].name = pc_fz[l].name = pc_bx[l].name = pc_by[l].name = "gemm_precond";
       if (precond_bf16) continue;  // the BF16 plans below replace them
       pc_fx[l].finalize(); pc_fz[l].finalize(); pc_bx[l].finalize(); pc_by[l].finalize();
     }
-    for (i64 l = 0; l <= levels; l++) {
-      pc_fcopy[l].finalize();
-      pc_bcopy[l].finalize();
-    }
+    for (i64 l = 0; l <= levels; l++) pc_fcopy[l].finalize();
     if (precond_bf16) build_bf16_plans(nr);
     pc_built = true;
   }
@@ -2391,11 +2452,10 @@ class Solver : public SolverBase {
       if (precond_bf16) {
         for (i64 l = levels; l >= 0; l--) {
           bf_fx[l].run(st());
-          pc_fcopy[l].run(st());
+          if (pc_fcopy[l].n) pc_fcopy[l].run(st());
           bf_fz[l].run(st());
         }
         for (i64 l = 0; l <= levels; l++) {
-          pc_bcopy[l].run(st());
           bf_bx[l].run(st());
           bf_by[l].run(st());
         }
@@ -2405,11 +2465,10 @@ class Solver : public SolverBase {
     }
     for (i64 l = levels; l >= 0; l--) {
       pc_fx[l].run(st());
-      pc_fcopy[l].run(st());
+      if (pc_fcopy[l].n) pc_fcopy[l].run(st());
       pc_fz[l].run(st());
     }
     for (i64 l = 0; l <= levels; l++) {
-      pc_bcopy[l].run(st());
       pc_bx[l].run(st());
       pc_by[l].run(st());
     }

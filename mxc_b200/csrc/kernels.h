@@ -144,6 +144,12 @@ template <typename T>
 cudaError_t launch_skinny_nn(int nr, int wide, const GemmTask<T>* d_tasks, const GemmEntry<T>* d_ents,
                              const int2* d_tiles, int ntiles, cudaStream_t st, int* bulk_err = nullptr);
 int skinny_rows_per_cta(int wide);
+// The same products by rows (k_apply.cu): one CTA per apply_rows_per_cta(rl)
+// rows of a task, rl = 1 or 2; both give the same bits.
+template <typename T>
+cudaError_t launch_apply(int nr, int rl, const GemmTask<T>* d_tasks, const GemmEntry<T>* d_ents, const int2* d_tiles,
+                         int ntiles, cudaStream_t st);
+int apply_rows_per_cta(int rl);
 // Reduction of a split task: dst (m x n, ld ldd) = beta dst + sum of `parts`
 // consecutive m x n partial results at src.
 template <typename T>
@@ -220,6 +226,8 @@ struct BfEntry {
   float alpha;
   const float* scale;
 };
+cudaError_t launch_apply_bf16(int nr, int rl, const GemmTask<float>* d_tasks, const BfEntry* d_ents,
+                              const int2* d_tiles, int ntiles, cudaStream_t st);
 cudaError_t launch_bf16_pack(const BfPackTask* d_tasks, int ntasks, cudaStream_t st);
 // 5-16 right-hand sides run on the BF16 tensor cores (k_stream_bf16_mma),
 // 1-4 on the FMA pipe.

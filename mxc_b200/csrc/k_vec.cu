@@ -53,25 +53,32 @@ cudaError_t launch_conj_interleaved(double* X, i64 n, i64 ld, int nrhs, cudaStre
 }
 
 constexpr int DOT_THREADS = 256;
-constexpr i64 DOT_ROWS = 8192;  // rows per chunk
-int dots_chunks(i64 n) { return (int)((n + DOT_ROWS - 1) / DOT_ROWS); }
+// Rows per chunk of a dot product (a CTA): 1,024, doubled until at most 64
+// chunks cover a column, so that a short column still spreads over CTAs and a
+// long one leaves the second pass little to add (chunks of 8,192 rows ran one
+// CTA per column up to that length: 8,192 complex rows, 8 columns, 51 us).
+__host__ __device__ inline i64 dots_rows(i64 n) {
+  i64 r = 1024;
+  while (r * 64 < n) r *= 2;
+  return r;
+}
+int dots_chunks(i64 n) { return (int)((n + dots_rows(n) - 1) / dots_rows(n)); }
 
 // partial[(g * kvec + j) * nrhs + c] = sum over rows of chunk g of V_j[:, c] * w[:, c]
 __global__ void __launch_bounds__(DOT_THREADS) k_dots_partial(const double* __restrict__ V, i64 vstride, int kvec,
                                                               const double* __restrict__ w, i64 n, int nrhs,
                                                               double* __restrict__ partial) {
   __shared__ double red[32];
-  const int g = blockIdx.x, c = blockIdx.y;
-  const i64 r0 = (i64)g * DOT_ROWS;
-  const i64 r1 = r0 + DOT_ROWS < n ? r0 + DOT_ROWS : n;
+  const int g = blockIdx.x, c = blockIdx.y, j = blockIdx.z;
+  const i64 rows = dots_rows(n), r0 = (i64)g * rows;
+  const i64 r1 = r0 + rows < n ? r0 + rows : n;
   const double* wc = w + (i64)c * n;
-  for (int j = 0; j < kvec; j++) {
-    const double* vc = V + (i64)j * vstride + (i64)c * n;
-    double s = 0.;
-    for (i64 r = r0 + threadIdx.x; r < r1; r += DOT_THREADS) s += vc[r] * wc[r];
-    s = BlockReduce<double>::sum(s, red);
-    if (threadIdx.x == 0) partial[((i64)g * kvec + j) * nrhs + c] = s;
-  }
+  const double* vc = V + (i64)j * vstride + (i64)c * n;
+  double s = 0.;
+#pragma unroll 4
+  for (i64 r = r0 + threadIdx.x; r < r1; r += DOT_THREADS) s += vc[r] * wc[r];
+  s = BlockReduce<double>::sum(s, red);
+  if (threadIdx.x == 0) partial[((i64)g * kvec + j) * nrhs + c] = s;
 }
 
 __global__ void k_dots_final(const double* __restrict__ partial, int nchunks, int kvec, int nrhs, double* __restrict__ out,
@@ -86,7 +93,7 @@ __global__ void k_dots_final(const double* __restrict__ partial, int nchunks, in
 
 cudaError_t launch_dots_strided(const double* V, i64 vstride, int kvec, const double* w, i64 n, int nrhs,
                                 double* partial, int nchunks, double* out, i64 ostride, cudaStream_t st) {
-  dim3 grid(nchunks, nrhs);
+  dim3 grid(nchunks, nrhs, kvec);
   note_launch();
   k_dots_partial<<<grid, DOT_THREADS, 0, st>>>(V, vstride, kvec, w, n, nrhs, partial);
   int tot = kvec * nrhs;
@@ -219,24 +226,23 @@ __global__ void __launch_bounds__(DOT_THREADS) k_cdots_partial(const double* __r
                                                                const double* __restrict__ w, i64 nc, int nrhs,
                                                                double* __restrict__ partial) {
   __shared__ double red[32];
-  const int g = blockIdx.x, c = blockIdx.y;
-  const i64 r0 = (i64)g * DOT_ROWS;
-  const i64 r1 = r0 + DOT_ROWS < nc ? r0 + DOT_ROWS : nc;
+  const int g = blockIdx.x, c = blockIdx.y, j = blockIdx.z;
+  const i64 rows = dots_rows(nc), r0 = (i64)g * rows;
+  const i64 r1 = r0 + rows < nc ? r0 + rows : nc;
   const double2* wc = reinterpret_cast<const double2*>(w) + (i64)c * nc;
-  for (int j = 0; j < kvec; j++) {
-    const double2* vc = reinterpret_cast<const double2*>(V + (i64)j * vstride) + (i64)c * nc;
-    double sr = 0., si = 0.;
-    for (i64 r = r0 + threadIdx.x; r < r1; r += DOT_THREADS) {
-      const double2 a = vc[r], b = wc[r];
-      sr += a.x * b.x + a.y * b.y;
-      si += a.x * b.y - a.y * b.x;
-    }
-    sr = BlockReduce<double>::sum(sr, red);
-    si = BlockReduce<double>::sum(si, red);
-    if (threadIdx.x == 0) {
-      partial[(((i64)g * kvec + j) * nrhs + c) * 2] = sr;
-      partial[(((i64)g * kvec + j) * nrhs + c) * 2 + 1] = si;
-    }
+  const double2* vc = reinterpret_cast<const double2*>(V + (i64)j * vstride) + (i64)c * nc;
+  double sr = 0., si = 0.;
+#pragma unroll 4
+  for (i64 r = r0 + threadIdx.x; r < r1; r += DOT_THREADS) {
+    const double2 a = vc[r], b = wc[r];
+    sr += a.x * b.x + a.y * b.y;
+    si += a.x * b.y - a.y * b.x;
+  }
+  sr = BlockReduce<double>::sum(sr, red);
+  si = BlockReduce<double>::sum(si, red);
+  if (threadIdx.x == 0) {
+    partial[(((i64)g * kvec + j) * nrhs + c) * 2] = sr;
+    partial[(((i64)g * kvec + j) * nrhs + c) * 2 + 1] = si;
   }
 }
 
@@ -254,12 +260,13 @@ __global__ void k_cdots_final(const double* __restrict__ partial, int nchunks, i
   out[(i64)c * ostride + 2 * j + 1] = si;
 }
 
-int cdots_chunks(i64 nc) { return (int)((nc + DOT_ROWS - 1) / DOT_ROWS); }
+// At most dots_chunks(2 nc), which sizes the partial sums.
+int cdots_chunks(i64 nc) { return dots_chunks(nc); }
 
 cudaError_t launch_cdots_strided(const double* V, i64 vstride, int kvec, const double* w, i64 nc, int nrhs,
                                  double* partial, int nchunks, double* out, i64 ostride, cudaStream_t st) {
   if ((reinterpret_cast<uintptr_t>(V) | reinterpret_cast<uintptr_t>(w)) & 15 || vstride % 2) return cudaErrorInvalidValue;
-  dim3 grid(nchunks, nrhs);
+  dim3 grid(nchunks, nrhs, kvec);
   note_launch();
   k_cdots_partial<<<grid, DOT_THREADS, 0, st>>>(V, vstride, kvec, w, nc, nrhs, partial);
   int tot = kvec * nrhs;

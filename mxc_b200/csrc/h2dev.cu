@@ -1410,9 +1410,10 @@ class Solver : public SolverBase {
           if (sketch) {
             // Y = Omega XF over the whole far list (k_sketch.cu), or XF
             // itself where the list has at most M bodies.
-            const int tm = sketch_tile_rows(), tn = sketch_tile_cols();
+            const int tm = sketch_tile_rows((int)lv.maxM), tn = sketch_tile_cols();
             std::vector<int4> tiles;
             double sfl = 0.;
+            i64 longest = 0;
             for (i64 i = 0; i < nodes; i++) {
               const i64 M = lv.dims[i], S = soff[i + 1] - soff[i];
               if (M == 0 || S == 0) continue;
@@ -1420,16 +1421,28 @@ class Solver : public SolverBase {
               for (i64 a = 0; a < (rows + tm - 1) / tm; a++)
                 for (i64 c = 0; c < (M + tn - 1) / tn; c++) tiles.push_back(make_int4((int)i, (int)a, (int)c, 0));
               if (S > M) sfl += 2. * (double)M * (double)M * (double)S;
+              longest = std::max(longest, S);
             }
+            const int parts = sketch_parts((i64)tiles.size(), tm, longest);
+            const size_t ntl = tiles.size();
+            for (int p = 1; p < parts; p++)
+              for (size_t z = 0; z < ntl; z++) tiles.push_back(make_int4(tiles[z].x, tiles[z].y, tiles[z].z, p));
             DVec<i64> d_roff, d_rstart, d_rend;
             DVec<int4> d_tiles;
+            DVec<double> Y;
             d_roff.upload(roff);
             d_rstart.upload(rstart);
             d_rend.upload(rend);
             d_tiles.upload(tiles);
+            double* y = reinterpret_cast<double*>(Rws.p);
+            if (parts > 1 || !std::is_same<T, double>::value) {
+              Y.alloc((size_t)parts * lv.qoff[nodes]);
+              y = Y.p;
+            }
             Prof pf("sketch", sfl, 24. * (double)soff[nodes]);
             ck(launch_sketch<T>(kp, bodies.p, lv.pts.p, lv.d_xoff.p, lv.d_dims.p, lv.d_qoff.p, d_roff.p, d_rstart.p,
-                                d_rend.p, d_tiles.p, (int)tiles.size(), Rws.p, st()),
+                                d_rend.p, d_tiles.p, (int)tiles.size(), tm, parts, lv.qoff[nodes], y, Rws.p,
+                                (int)nodes, st()),
                "sketch");
           } else {
             Prof pf("sample_tsqr", fl, (double)sidx.size() * 28.);

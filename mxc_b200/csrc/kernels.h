@@ -33,13 +33,17 @@ cudaError_t launch_sample_tsqr(const KernelParams& kp, const double* bodies, con
                                int nboxes, int maxM, cudaStream_t st);
 // Full-far-field sketch (k_sketch.cu): Rws[box] (row-major M x M) = Omega XF
 // over every far body (ranges roff[box]..roff[box+1]-1 of rstart / rend), or
-// the first S rows = XF when S <= M.  tiles: {box, row tile, column tile}.
+// the first S rows = XF when S <= M.  tiles: {box, row tile, column tile, part}
+// for every part of 0..parts-1; Y: the parts' sums, pstride doubles apart
+// (FP64 with one part: Rws itself).
 template <typename T>
 cudaError_t launch_sketch(const KernelParams& kp, const double* bodies, const double* pts, const i64* xoff,
                           const i64* dims, const i64* qoff, const i64* roff, const i64* rstart, const i64* rend,
-                          const int4* d_tiles, int ntiles, T* Rws, cudaStream_t st);
-int sketch_tile_rows();
+                          const int4* d_tiles, int ntiles, int tile_rows, int parts, i64 pstride, double* Y, T* Rws,
+                          int nboxes, cudaStream_t st);
+int sketch_tile_rows(int M);
 int sketch_tile_cols();
+int sketch_parts(i64 tiles, int tile_rows, i64 bodies);
 template <typename T>
 cudaError_t launch_cpqr(const i64* dims, const i64* krows, T* Rws, const i64* qoff, int* perm, const i64* xoff,
                         double* maxpiv, int* nonzero, i64 step_cap, double epi, int nboxes, int maxM, cudaStream_t st);

@@ -54,3 +54,25 @@ def test_operator_box_sizes(handle, box, eps):
     A.matVecMul(y)
     d = m.dense_matvec(handle, k, b, x)
     assert np.linalg.norm(y - d) < 10 * eps * np.linalg.norm(d)
+
+
+@pytest.mark.parametrize("box,seed", [(20, 1), (64, 2), (130, 3), (321, 4)])
+@pytest.mark.parametrize("precision", [m.FP64, m.FP32])
+def test_sketched_operator_box_sizes(box, seed, precision):
+    """Sketched bases at row-tile counts, far lists cut into parts and boxes that
+    take their whole far block: the product is within a hundred times the
+    threshold of the dense one (the sketch's distortion, FP32 rounding)."""
+    n = 16 * box
+    b = np.random.default_rng(seed).random((n, 3))
+    t = m.build_tree(b, 4)
+    h = m.Handle(0)
+    h.set_option(m._lib.OPT_SAMPLING, m._lib.SAMPLING_SKETCH)
+    eps = 1e-9 if precision == m.FP64 else 1e-4
+    A = m.H2MatrixSolver(h, m.Laplace3D(1e-2), eps, 100, 0, t, 1.0, b, precision=precision)
+    x = np.random.default_rng(2).random(n)
+    y = x.copy()
+    A.matVecMul(y)
+    d = m.dense_matvec(h, m.Laplace3D(1e-2), b, x)
+    assert np.linalg.norm(y - d) < 100 * eps * np.linalg.norm(d)
+    A.close()
+    h.close()

@@ -761,10 +761,16 @@ __global__ void __launch_bounds__(128) k_pivchol_update(const i64* __restrict__ 
 #pragma unroll
       for (int i = 0; i < 4; i++) {
         const int r = r0 + wm * 32 + i * 8 + fr, c = c0 + wn * 32 + j * 8 + 2 * fk + h;
-        if (r < M && c < M) {
-          double* p = g + r + (i64)c * M;
-          *p = *p + acc[i][j][h];
-        }
+        if (r < M && c < M) acc[i][j][h] = g[r + (i64)c * M] + acc[i][j][h];
+      }
+#pragma unroll
+  for (int j = 0; j < 4; j++)
+#pragma unroll
+    for (int h = 0; h < 2; h++)
+#pragma unroll
+      for (int i = 0; i < 4; i++) {
+        const int r = r0 + wm * 32 + i * 8 + fr, c = c0 + wn * 32 + j * 8 + 2 * fk + h;
+        if (r < M && c < M) g[r + (i64)c * M] = acc[i][j][h];
       }
 }
 
@@ -1229,10 +1235,16 @@ __global__ void __launch_bounds__(256) k_qr_update(const QrPanelTask<T>* __restr
 #pragma unroll
           for (int i = 0; i < 2; i++) {
             const int r = r0 + 8 * i + fr, c = 8 * j + 2 * fk + h;
-            if (r < m && c < nc) {
-              double* p = A + r + (i64)c * t.M;
-              *p = *p + acc[i][j][h];
-            }
+            if (r < m && c < nc) acc[i][j][h] = A[r + (i64)c * t.M] + acc[i][j][h];
+          }
+#pragma unroll
+      for (int j = 0; j < 4; j++)
+#pragma unroll
+        for (int h = 0; h < 2; h++)
+#pragma unroll
+          for (int i = 0; i < 2; i++) {
+            const int r = r0 + 8 * i + fr, c = 8 * j + 2 * fk + h;
+            if (r < m && c < nc) A[r + (i64)c * t.M] = acc[i][j][h];
           }
     }
   } else {

@@ -151,6 +151,15 @@ __global__ void __launch_bounds__(BM / 2) k_stream_bf16(const GemmTask<float>* _
     slot = (slot + 1) % BF_ST;
   }
   bf_wait<0>();
+  // beta C first, so that its loads are all in flight before the first store
+  // (interleaved with the stores each waited for the one before).
+  if (task.beta != 0.f)
+#pragma unroll
+    for (int t = 0; t < 2; t++)
+#pragma unroll
+      for (int j = 0; j < NR; j++)
+        if (2 * tid + t < mrows && j < task.n)
+          acc[t][j] = task.beta * task.C[(m0 + 2 * tid + t) + (i64)j * task.ldc] + acc[t][j];
 #pragma unroll
   for (int t = 0; t < 2; t++) {
     const int r = 2 * tid + t;
@@ -158,8 +167,7 @@ __global__ void __launch_bounds__(BM / 2) k_stream_bf16(const GemmTask<float>* _
 #pragma unroll
     for (int j = 0; j < NR; j++) {
       if (j >= task.n) break;
-      float* p = task.C + (m0 + r) + (i64)j * task.ldc;
-      *p = (task.beta == 0.f) ? acc[t][j] : task.beta * (*p) + acc[t][j];
+      task.C[(m0 + r) + (i64)j * task.ldc] = acc[t][j];
     }
   }
 }
@@ -311,6 +319,19 @@ __global__ void __launch_bounds__(BFM_BM, 2) k_stream_bf16_mma(const GemmTask<fl
   if (!live) return;
   // C fragment of block rb: c[2h + q] is MMA row g8 + 8h = tile row
   // 4 g8 + 2 rb + h, column 2 t4 + q of the column block.
+  if (task.beta != 0.f)
+#pragma unroll
+    for (int rb = 0; rb < 2; rb++)
+#pragma unroll
+      for (int h = 0; h < 2; h++)
+#pragma unroll
+        for (int cb = 0; cb < NF; cb++)
+#pragma unroll
+          for (int q = 0; q < 2; q++) {
+            const int r = wr + 4 * g8 + 2 * rb + h, c = cb * 8 + 2 * t4 + q;
+            if (r < mrows && c < task.n)
+              acc[rb][cb][2 * h + q] = task.beta * task.C[(m0 + r) + (i64)c * task.ldc] + acc[rb][cb][2 * h + q];
+          }
 #pragma unroll
   for (int rb = 0; rb < 2; rb++)
 #pragma unroll
@@ -322,11 +343,7 @@ __global__ void __launch_bounds__(BFM_BM, 2) k_stream_bf16_mma(const GemmTask<fl
 #pragma unroll
         for (int q = 0; q < 2; q++) {
           const int c = cb * 8 + 2 * t4 + q;
-          if (c < task.n) {
-            float* p = task.C + (m0 + r) + (i64)c * task.ldc;
-            const float v = acc[rb][cb][2 * h + q];
-            *p = (task.beta == 0.f) ? v : task.beta * (*p) + v;
-          }
+          if (c < task.n) task.C[(m0 + r) + (i64)c * task.ldc] = acc[rb][cb][2 * h + q];
         }
     }
 }

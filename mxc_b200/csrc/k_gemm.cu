@@ -342,6 +342,15 @@ __global__ void __launch_bounds__(BM / 2, 1024 / BM) k_stream_nn(const GemmTask<
     slot = (slot + 1) % ST;
   }
   cp_async_wait<0>();
+  // beta C first, so that its loads are all in flight before the first store
+  // (interleaved with the stores each waited for the one before).
+  if (task.beta != T(0))
+#pragma unroll
+    for (int t = 0; t < 2; t++)
+#pragma unroll
+      for (int j = 0; j < NR; j++)
+        if (2 * tid + t < mrows && j < task.n)
+          acc[t][j] = task.beta * task.C[(m0 + 2 * tid + t) + (i64)j * task.ldc] + acc[t][j];
 #pragma unroll
   for (int t = 0; t < 2; t++) {
     const int r = 2 * tid + t;
@@ -349,8 +358,7 @@ __global__ void __launch_bounds__(BM / 2, 1024 / BM) k_stream_nn(const GemmTask<
 #pragma unroll
     for (int j = 0; j < NR; j++) {
       if (j >= task.n) break;
-      T* p = task.C + (m0 + r) + (i64)j * task.ldc;
-      *p = (task.beta == T(0)) ? acc[t][j] : task.beta * (*p) + acc[t][j];
+      task.C[(m0 + r) + (i64)j * task.ldc] = acc[t][j];
     }
   }
 }
@@ -476,6 +484,16 @@ __global__ void __launch_bounds__(BM, BM == 256 ? 3 : 6)
   }
   cp_async_wait<0>();
   // D fragment: lane holds row lane >> 2, columns 2 (lane & 3) + {0, 1}.
+  if (task.beta != 0.)  // as k_stream_nn
+#pragma unroll
+    for (int i = 0; i < 4; i++)
+#pragma unroll
+      for (int j = 0; j < NF; j++)
+#pragma unroll
+        for (int h = 0; h < 2; h++) {
+          const int r = warp * 32 + i * 8 + fr, c = j * 8 + 2 * fk + h;
+          if (r < mrows && c < task.n) acc[i][j][h] = task.beta * task.C[(m0 + r) + (i64)c * task.ldc] + acc[i][j][h];
+        }
 #pragma unroll
   for (int i = 0; i < 4; i++) {
     const int r = warp * 32 + i * 8 + fr;
@@ -485,10 +503,7 @@ __global__ void __launch_bounds__(BM, BM == 256 ? 3 : 6)
 #pragma unroll
       for (int h = 0; h < 2; h++) {
         const int c = j * 8 + 2 * fk + h;
-        if (c < task.n) {
-          double* p = task.C + (m0 + r) + (i64)c * task.ldc;
-          *p = (task.beta == 0.) ? acc[i][j][h] : task.beta * (*p) + acc[i][j][h];
-        }
+        if (c < task.n) task.C[(m0 + r) + (i64)c * task.ldc] = acc[i][j][h];
       }
   }
 }
@@ -725,6 +740,19 @@ __global__ void __launch_bounds__(BM + 32) k_stream_dtma(const GemmTask<double>*
   if (!ok) return;
   // D fragment of 16-row block rb: c[2h + q] is MMA row g8 + 8h (tile row
   // 2 g8 + h of the block), column 2 t4 + q of the column block.
+  if (task.beta != 0.)  // as k_stream_nn
+#pragma unroll
+    for (int rb = 0; rb < 2; rb++)
+#pragma unroll
+      for (int h = 0; h < 2; h++)
+#pragma unroll
+        for (int cb = 0; cb < NF; cb++)
+#pragma unroll
+          for (int q = 0; q < 2; q++) {
+            const int r = wr + 16 * rb + 2 * g8 + h, c = cb * 8 + 2 * t4 + q;
+            if (r < mrows && c < task.n)
+              acc[rb][cb][2 * h + q] = task.beta * task.C[(m0 + r) + (i64)c * task.ldc] + acc[rb][cb][2 * h + q];
+          }
 #pragma unroll
   for (int rb = 0; rb < 2; rb++)
 #pragma unroll
@@ -736,10 +764,7 @@ __global__ void __launch_bounds__(BM + 32) k_stream_dtma(const GemmTask<double>*
 #pragma unroll
         for (int q = 0; q < 2; q++) {
           const int c = cb * 8 + 2 * t4 + q;
-          if (c < task.n) {
-            double* p = task.C + (m0 + r) + (i64)c * task.ldc;
-            *p = (task.beta == 0.) ? acc[rb][cb][2 * h + q] : task.beta * (*p) + acc[rb][cb][2 * h + q];
-          }
+          if (c < task.n) task.C[(m0 + r) + (i64)c * task.ldc] = acc[rb][cb][2 * h + q];
         }
     }
 }
@@ -894,6 +919,19 @@ __global__ void __launch_bounds__(BM, BM == 256 ? 3 : 6)
   }
   cp_async_wait<0>();
   // C fragment: c0 (g, 2t), c1 (g, 2t + 1), c2 (g + 8, 2t), c3 (g + 8, 2t + 1).
+  if (task.beta != 0.f)  // as k_stream_nn
+#pragma unroll
+    for (int i = 0; i < 2; i++)
+#pragma unroll
+      for (int hh = 0; hh < 2; hh++)
+#pragma unroll
+        for (int j = 0; j < NF; j++)
+#pragma unroll
+          for (int q = 0; q < 2; q++) {
+            const int r = warp * 32 + i * 16 + g + 8 * hh, c = j * 8 + 2 * t4 + q;
+            if (r < mrows && c < task.n)
+              acc[i][j][2 * hh + q] = task.beta * task.C[(m0 + r) + (i64)c * task.ldc] + acc[i][j][2 * hh + q];
+          }
 #pragma unroll
   for (int i = 0; i < 2; i++)
 #pragma unroll
@@ -905,11 +943,7 @@ __global__ void __launch_bounds__(BM, BM == 256 ? 3 : 6)
 #pragma unroll
         for (int q = 0; q < 2; q++) {
           const int c = j * 8 + 2 * t4 + q;
-          if (c < task.n) {
-            float* p = task.C + (m0 + r) + (i64)c * task.ldc;
-            const float v = acc[i][j][2 * hh + q];
-            *p = (task.beta == 0.f) ? v : task.beta * (*p) + v;
-          }
+          if (c < task.n) task.C[(m0 + r) + (i64)c * task.ldc] = acc[i][j][2 * hh + q];
         }
     }
 }

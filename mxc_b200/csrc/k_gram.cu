@@ -325,6 +325,19 @@ __global__ void __launch_bounds__(DG_NT, 3) k_dgemm(const GemmTask<double>* __re
   }
   gwait<0>();
   // D fragment of m8n8k4: lane holds row lane >> 2, columns 2 (lane & 3) + {0, 1}.
+  // beta C first, so that its loads are all in flight before the first store
+  // (interleaved with the stores each waited for the one before).
+  if (task.beta != 0.)
+#pragma unroll
+    for (int i = 0; i < 4; i++)
+#pragma unroll
+      for (int j = 0; j < 4; j++)
+#pragma unroll
+        for (int h = 0; h < 2; h++) {
+          const int r = wm * 32 + i * 8 + fr, c = wn * 32 + j * 8 + 2 * fk + h;
+          if (r < mrows && c < ncols)
+            acc[i][j][h] = task.beta * task.C[(i64)(m0 + r) + (i64)(n0 + c) * task.ldc] + acc[i][j][h];
+        }
 #pragma unroll
   for (int i = 0; i < 4; i++) {
     const int r = wm * 32 + i * 8 + fr;
@@ -334,10 +347,7 @@ __global__ void __launch_bounds__(DG_NT, 3) k_dgemm(const GemmTask<double>* __re
 #pragma unroll
       for (int h = 0; h < 2; h++) {
         const int c = wn * 32 + j * 8 + 2 * fk + h;
-        if (c < ncols) {
-          double* p = task.C + (i64)(m0 + r) + (i64)(n0 + c) * task.ldc;
-          *p = (task.beta == 0.) ? acc[i][j][h] : task.beta * (*p) + acc[i][j][h];
-        }
+        if (c < ncols) task.C[(i64)(m0 + r) + (i64)(n0 + c) * task.ldc] = acc[i][j][h];
       }
   }
 }

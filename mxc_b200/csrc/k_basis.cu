@@ -1313,25 +1313,28 @@ namespace h2b {
 // After the blocked QR of W (M x rank): R's slot gets triu(W[:rank, :rank]),
 // W becomes the explicit unit lower-trapezoidal V, Q the identity (for the
 // compact-WY formation that follows).
+// gridDim.y CTAs per box, each its own columns.
 template <typename T>
 __global__ void __launch_bounds__(256) k_qr_extract(const QrExtractTask<T>* __restrict__ tasks) {
   const QrExtractTask<T> t = tasks[blockIdx.x];
-  const int M = t.M, r = t.rank;
-  for_each_rc(M, M, [&](int i, int c, int e) {
-    t.R[e] = (c < r && i <= c) ? t.W[i + (i64)c * M] : T(0);
-    t.Q[e] = i == c ? T(1) : T(0);
-  });
-  __syncthreads();
-  for_each_rc(M, r, [&](int i, int c, int e) {
-    if (i <= c) t.W[e] = i == c ? T(1) : T(0);
-  });
+  const int M = t.M, r = t.rank, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  for (int c = blockIdx.y * 8 + warp; c < M; c += gridDim.y * 8) {
+    const i64 o = (i64)c * M;
+#pragma unroll 4
+    for (int i = lane; i < M; i += 32) {
+      const T w = c < r ? t.W[o + i] : T(0);
+      t.R[o + i] = (c < r && i <= c) ? w : T(0);
+      t.Q[o + i] = i == c ? T(1) : T(0);
+      if (c < r && i <= c) t.W[o + i] = i == c ? T(1) : T(0);
+    }
+  }
 }
 
 template <typename T>
 cudaError_t launch_qr_extract(const QrExtractTask<T>* d_tasks, int ntasks, cudaStream_t st) {
   if (ntasks == 0) return cudaSuccess;
   note_launch();
-  k_qr_extract<T><<<ntasks, 256, 0, st>>>(d_tasks);
+  k_qr_extract<T><<<dim3(ntasks, 8), 256, 0, st>>>(d_tasks);
   return cudaGetLastError();
 }
 template cudaError_t launch_qr_extract<double>(const QrExtractTask<double>*, int, cudaStream_t);

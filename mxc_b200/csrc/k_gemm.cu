@@ -112,62 +112,63 @@ template cudaError_t launch_seg_gemm<double>(int, const GemmTask<double>*, const
 template cudaError_t launch_seg_gemm<float>(int, const GemmTask<float>*, const GemmEntry<float>*, const TileRef*, int,
                                             cudaStream_t);
 
-// One CTA per entry: dst (m x n, ld ldd) = src or src^T (ld lds).  Plain
-// copies walk the elements column by column (consecutive threads on
-// consecutive rows, one division per thread, none per element); transposed
-// copies go through 32 x 32 shared-memory tiles so that both the reads of
-// src and the writes of dst are coalesced.
+// dst (m x n, ld ldd) = src or src^T (ld lds), gridDim.y CTAs per entry.  Plain
+// copies: columns dealt to the CTAs' warps, consecutive lanes on consecutive
+// rows; transposed copies: 32 x 32 tiles through shared memory, so that both
+// the reads of src and the writes of dst are coalesced.  One CTA per entry left
+// most SMs idle on the upper levels and walked a box's 64 tiles one barrier
+// pair at a time (256 transposes of 256 x 256 FP32: 175 us).
 template <typename T>
 __global__ void __launch_bounds__(256) k_batched_copy(const CopyEntry<T>* __restrict__ ents) {
   const CopyEntry<T> e = ents[blockIdx.x];
   const int m = e.m, n = e.n;
   if (m <= 0 || n <= 0) return;
+  const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
   if (!e.trans) {
-    if ((i64)m * n < ((i64)1 << 31)) {
-      const int stride = (int)blockDim.x, dq = stride / m, dr = stride - dq * m, total = m * n;
-      int x = (int)threadIdx.x;
-      int c = x / m, r = x - c * m;
-      for (; x < total; x += stride) {
-        e.dst[r + (i64)c * e.ldd] = e.src[r + (i64)c * e.lds];
-        r += dr;
-        c += dq;
-        if (r >= m) {
-          r -= m;
-          c++;
-        }
-      }
-    } else {
-      for (i64 x = threadIdx.x; x < (i64)m * n; x += blockDim.x) {
-        const int r = (int)(x % m), c = (int)(x / m);
-        e.dst[r + (i64)c * e.ldd] = e.src[r + (i64)c * e.lds];
-      }
+    if (n == 1) {
+      for (int r = blockIdx.y * 256 + threadIdx.x; r < m; r += gridDim.y * 256) e.dst[r] = e.src[r];
+      return;
+    }
+    for (int c = blockIdx.y * 8 + ty; c < n; c += gridDim.y * 8) {
+      const T* s = e.src + (i64)c * e.lds;
+      T* d = e.dst + (i64)c * e.ldd;
+#pragma unroll 4
+      for (int r = tx; r < m; r += 32) d[r] = s[r];
     }
     return;
   }
   // dst(r, c) = src(c, r): the tile at dst rows r0.., columns c0.. is the
   // tile at src rows c0.., columns r0...
   __shared__ T tile[32][33];
-  const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;  // 8 rows of 32 per pass
-  for (int c0 = 0; c0 < n; c0 += 32)
-    for (int r0 = 0; r0 < m; r0 += 32) {
-      for (int i = ty; i < 32; i += 8) {
-        const int sr = c0 + tx, sc = r0 + i;  // src(sr, sc) = dst(sc, sr)
-        tile[i][tx] = (sr < n && sc < m) ? e.src[sr + (i64)sc * e.lds] : T(0);
-      }
-      __syncthreads();
-      for (int i = ty; i < 32; i += 8) {
-        const int dr = r0 + tx, dc = c0 + i;
-        if (dr < m && dc < n) e.dst[dr + (i64)dc * e.ldd] = tile[tx][i];
-      }
-      __syncthreads();
+  const int tr = (m + 31) / 32, tiles = tr * ((n + 31) / 32);
+  for (int t = blockIdx.y; t < tiles; t += gridDim.y) {
+    const int r0 = t % tr * 32, c0 = t / tr * 32;
+    T v[4];
+#pragma unroll
+    for (int i = 0; i < 4; i++) {
+      const int sr = c0 + tx, sc = r0 + ty + 8 * i;  // src(sr, sc) = dst(sc, sr)
+      v[i] = (sr < n && sc < m) ? e.src[sr + (i64)sc * e.lds] : T(0);
     }
+#pragma unroll
+    for (int i = 0; i < 4; i++) tile[ty + 8 * i][tx] = v[i];
+    __syncthreads();
+#pragma unroll
+    for (int i = 0; i < 4; i++) {
+      const int dr = r0 + tx, dc = c0 + ty + 8 * i;
+      if (dr < m && dc < n) e.dst[dr + (i64)dc * e.ldd] = tile[tx][ty + 8 * i];
+    }
+    __syncthreads();
+  }
 }
 
 template <typename T>
 cudaError_t launch_batched_copy(const CopyEntry<T>* d_ents, int n, cudaStream_t st) {
   if (n == 0) return cudaSuccess;
   note_launch();
-  k_batched_copy<T><<<n, 256, 0, st>>>(d_ents);
+  // About eight CTAs per SM, as many as a 256 x 256 block has tiles to share.
+  int y = 8 * 148 / n;
+  y = y < 4 ? 4 : y > 16 ? 16 : y;
+  k_batched_copy<T><<<dim3(n, y), 256, 0, st>>>(d_ents);
   return cudaGetLastError();
 }
 template cudaError_t launch_batched_copy<double>(const CopyEntry<double>*, int, cudaStream_t);

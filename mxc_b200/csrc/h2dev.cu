@@ -405,14 +405,48 @@ static bool apply_by_rows(int nr, const std::vector<TK>& tasks, const std::vecto
   return rowtiles <= 256. && longest <= 512;
 }
 
+// Several host arrays in one device block, uploaded by one copy: a level of few
+// boxes runs its kernels in about the time that one upload takes the host, so a
+// plan's tasks, entries and tiles go together.
+struct PackedUpload {
+  std::vector<char> host;
+  DVec<char> dev;
+  template <typename X>
+  size_t add(const std::vector<X>& v) {
+    const size_t at = (host.size() + 255) / 256 * 256;
+    host.resize(at + v.size() * sizeof(X));
+    if (!v.empty()) std::memcpy(host.data() + at, v.data(), v.size() * sizeof(X));
+    return at;
+  }
+  void upload() {
+    dev.upload(host);
+    host.clear();
+    host.shrink_to_fit();
+  }
+  template <typename X>
+  X* at(size_t off) const { return reinterpret_cast<X*>(dev.p + off); }
+};
+// Part of a packed upload.
+template <typename X>
+struct DView {
+  X* p = nullptr;
+  size_t n = 0, off = 0;
+  void put(PackedUpload& u, const std::vector<X>& v) {
+    off = u.add(v);
+    n = v.size();
+  }
+  void bind(const PackedUpload& u) { p = n ? u.at<X>(off) : nullptr; }
+};
+
 // Host-built list of segmented-GEMM tasks, uploaded once and replayed.
 template <typename T>
 struct GemmPlan {
   std::vector<GemmTask<T>> tasks;
   std::vector<GemmEntry<T>> ents;
-  DVec<GemmTask<T>> d_tasks;
-  DVec<GemmEntry<T>> d_ents;
-  DVec<TileRef> d_tiles;
+  PackedUpload packed;
+  DView<GemmTask<T>> d_tasks;
+  DView<GemmEntry<T>> d_ents;
+  DView<TileRef> d_tiles;
   int ntiles = 0;
   int shape = GEMM_BIG;
   int tc_mode = 0;  // GEMM_TC: 1 three-term TF32 split, 2 single TF32
@@ -420,11 +454,11 @@ struct GemmPlan {
   double flops = 0., bytes = 0.;  // algorithmic work of one run
   bool skinny_nn = false;          // use k_skinny_nn instead of the tiled kernel
   int nr = 0;
-  DVec<int2> d_rtiles, d_rtiles_w;  // row tiles of the 128- and 256-row streaming variants
+  DView<int2> d_rtiles, d_rtiles_w;  // row tiles of the 128- and 256-row streaming variants
   // Autotuned tilings of the streaming path: 0 = per-task rule (256-row
   // tiles where they pad no more than 128-row ones), 1 = all 128-row, 2 =
   // all 256-row tiles.
-  DVec<int2> d_alt_n, d_alt_w;
+  DView<int2> d_alt_n, d_alt_w;
   std::string tkey;
   mutable int variant = -1;
   // Only plans that overwrite their outputs (every beta zero) are timed:
@@ -484,8 +518,8 @@ struct GemmPlan {
         rows += t.m;
         for (int e = t.e0; e < t.e1; e++) elems += (double)t.m * ents[e].k;
       }
-      d_rtiles.upload(rt[0]);
-      d_rtiles_w.upload(rt[1]);
+      d_rtiles.put(packed, rt[0]);
+      d_rtiles_w.put(packed, rt[1]);
       tkey = tune_key(name, (int)sizeof(T), nr, (double)tasks.size(), rows, elems);
     }
     if (skinny_nn && !by_rows) split_tasks();
@@ -510,10 +544,10 @@ struct GemmPlan {
         rows += t.m;
         for (int e = t.e0; e < t.e1; e++) elems += (double)t.m * ents[e].k;
       }
-      d_rtiles.upload(rt[0]);
-      d_rtiles_w.upload(rt[1]);
-      d_alt_n.upload(alt[0]);
-      d_alt_w.upload(alt[1]);
+      d_rtiles.put(packed, rt[0]);
+      d_rtiles_w.put(packed, rt[1]);
+      d_alt_n.put(packed, alt[0]);
+      d_alt_w.put(packed, alt[1]);
       tkey = tune_key(name, (int)sizeof(T), nr, (double)tasks.size(), rows, elems);
       bulk_ok = sizeof(T) == 8 && nr > 4;
       for (const auto& e : ents)
@@ -522,7 +556,7 @@ struct GemmPlan {
     int bm = shape == GEMM_TC ? tc_gemm_tile() : gemm_tile_m(shape);
     int bn = shape == GEMM_TC ? tc_gemm_tile() : gemm_tile_n(shape);
     std::vector<TileRef> tiles;
-    for (int ti = 0; ti < (int)tasks.size(); ti++) {
+    for (int ti = 0; ti < (int)tasks.size() && !skinny_nn; ti++) {  // streaming plans have their own
       const auto& t = tasks[ti];
       if (t.m <= 0 || t.n <= 0) continue;
       if (t.e0 == t.e1 && t.beta == T(1)) continue;  // nothing to do
@@ -540,9 +574,14 @@ struct GemmPlan {
       }
     }
     bytes += sum_bytes;
-    d_tasks.upload(tasks);
-    d_ents.upload(ents);
-    d_tiles.upload(tiles);
+    d_tasks.put(packed, tasks);
+    d_ents.put(packed, ents);
+    d_tiles.put(packed, tiles);
+    packed.upload();
+    d_tasks.bind(packed);
+    d_ents.bind(packed);
+    d_tiles.bind(packed);
+    for (auto* v : {&d_rtiles, &d_rtiles_w, &d_alt_n, &d_alt_w}) v->bind(packed);
     tasks.clear();
     tasks.shrink_to_fit();
     ents.clear();
@@ -659,12 +698,12 @@ struct GemmPlan {
 
   void run_skinny(int v, cudaStream_t st) const {
     if (by_rows) {
-      const DVec<int2>& t = v == 0 ? d_rtiles_w : d_rtiles;
+      const DView<int2>& t = v == 0 ? d_rtiles_w : d_rtiles;
       ck(launch_apply<T>(nr, v == 0 ? 2 : 1, d_tasks.p, d_ents.p, t.p, (int)t.n, st), "apply");
       return;
     }
-    const DVec<int2>& w = v == 0 ? d_rtiles_w : d_alt_w;
-    const DVec<int2>& n = v == 0 ? d_rtiles : d_alt_n;
+    const DView<int2>& w = v == 0 ? d_rtiles_w : d_alt_w;
+    const DView<int2>& n = v == 0 ? d_rtiles : d_alt_n;
     int* be = (bulk_ok && g_cur) ? g_cur->d_tc_err : nullptr;
     if (be) g_cur->tc_pending = true;
     if (v != 1) ck(launch_skinny_nn<T>(nr, 1, d_tasks.p, d_ents.p, w.p, (int)w.n, st, be), "skinny_nn");

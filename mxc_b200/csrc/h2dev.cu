@@ -1462,7 +1462,9 @@ class Solver : public SolverBase {
               if (S > M) sfl += 2. * (double)M * (double)M * (double)S;
               longest = std::max(longest, S);
             }
-            const int parts = sketch_parts((i64)tiles.size(), tm, longest);
+            // The parts' sums take at most 512 MB beside the level's own blocks.
+            int parts = sketch_parts((i64)tiles.size(), tm, longest);
+            while (parts > 1 && (i64)parts * lv.qoff[nodes] > ((i64)1 << 26)) parts--;
             const size_t ntl = tiles.size();
             for (int p = 1; p < parts; p++)
               for (size_t z = 0; z < ntl; z++) tiles.push_back(make_int4(tiles[z].x, tiles[z].y, tiles[z].z, p));

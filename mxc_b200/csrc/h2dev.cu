@@ -820,7 +820,7 @@ struct MfPlan {
 
 // BF16 substitution plan: the tasks of one FP32 GemmPlan with each entry's
 // block packed to BF16 (per-block power-of-two scale), applied by
-// k_stream_bf16.
+// k_stream_bf16_mma, or by rows (k_apply).
 struct BfPlan {
   std::vector<GemmTask<float>> tasks;
   std::vector<BfEntry> ents;

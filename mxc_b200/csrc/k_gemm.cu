@@ -196,19 +196,16 @@ template cudaError_t launch_set_identity<float>(float*, const i64*, const i64*, 
 
 namespace h2b {
 
-// Multi-right-hand-side block-sparse apply: C_task (m x n, n <= NR) =
-// beta C + sum_e alpha_e A_e B_e with A_e and B_e as stored (column-major).
-// This is the shape of every H^2 matvec pass and every ULV substitution
-// step except the transposed ones, and it is bound by streaming A from HBM
-// once.  One CTA (BM / 2 threads) covers BM = 128 or 256 rows of a task
-// (tasks of at most 128 rows take the narrow variant).  The (entry, k-slab)
-// sequence of the task is one stream of stages: each stage is a BM x KS
-// slab of A and the KS x NR slab of B, copied by cp.async into a
+// Multi-right-hand-side block-sparse apply for 5 to 16 right-hand sides: C_task
+// (m x n) = beta C + sum_e alpha_e A_e B_e with A_e and B_e as stored
+// (column-major), bound by streaming A from HBM once (fewer columns and short
+// sums: k_apply.cu).  One CTA covers BM = 128 or 256 rows of a task.  The
+// (entry, k-slab) sequence of the task is one stream of stages: each stage is a
+// BM x KS slab of A and the KS x NR slab of B, copied by cp.async into an
 // ST-deep shared-memory ring (16-byte copies where the column starts are
 // 16-byte aligned, element copies otherwise; rows past m and k past K are
-// zero-filled), so ST-1 slabs are in flight while one is multiplied.  Each
-// thread owns two adjacent rows and all NR columns; B rows are read as
-// shared-memory broadcasts.  alpha_e != 1 scales the B slab in place.
+// zero-filled), so ST-1 slabs are in flight while one is multiplied.  alpha_e !=
+// 1 scales the B slab in place.
 __device__ __forceinline__ unsigned smem_u32(const void* p) { return (unsigned)__cvta_generic_to_shared(p); }
 __device__ __forceinline__ void cp_async_16(void* dst, const void* src, int src_bytes) {
   asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"(smem_u32(dst)), "l"(src), "r"(src_bytes));
@@ -222,152 +219,9 @@ __device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commi
 template <int N>
 __device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_group %0;\n" ::"n"(N)); }
 
-template <typename T>
-struct StreamCfg;
-template <>
-struct StreamCfg<double> { static constexpr int KS = 8, ST = 3; };
-template <>
-struct StreamCfg<float> { static constexpr int KS = 16, ST = 3; };
-
-template <typename T, int NR, int BM>
-constexpr size_t stream_smem() {
-  return sizeof(T) * (size_t)StreamCfg<T>::ST * StreamCfg<T>::KS * (BM + NR);
-}
-
-template <typename T, int NR, int BM>
-__global__ void __launch_bounds__(BM / 2, 1024 / BM) k_stream_nn(const GemmTask<T>* __restrict__ tasks,
-                                                      const GemmEntry<T>* __restrict__ ents,
-                                                      const int2* __restrict__ tiles) {
-  constexpr int KS = StreamCfg<T>::KS, ST = StreamCfg<T>::ST, NT = BM / 2;
-  constexpr int V = 16 / sizeof(T);  // elements per 16-byte copy
-  extern __shared__ __align__(16) unsigned char smem_raw[];
-  T* As = reinterpret_cast<T*>(smem_raw);  // [ST][KS][BM]
-  T* Bs = As + (size_t)ST * KS * BM;       // [ST][KS][NR]
-  const int2 tl = tiles[blockIdx.x];
-  const GemmTask<T> task = tasks[tl.x];
-  const int m0 = tl.y * BM;
-  const int mrows = min(BM, task.m - m0);
-  const int tid = threadIdx.x;
-
-  // Producer cursor: next (entry, k0) to stage.
-  int pe = task.e0, pk = 0;
-  while (pe < task.e1 && ents[pe].k <= 0) pe++;
-  auto issue = [&](int slot) {
-    if (pe < task.e1) {
-      const GemmEntry<T> en = ents[pe];
-      T* as = As + (size_t)slot * KS * BM;
-      T* bs = Bs + (size_t)slot * KS * NR;
-      const bool vec = ((reinterpret_cast<uintptr_t>(en.A) & 15) == 0) && (en.lda % V == 0);
-      if (vec) {
-        for (int c = tid; c < KS * (BM / V); c += NT) {
-          const int k = c / (BM / V), r = (c % (BM / V)) * V;
-          int valid = mrows - r;
-          valid = valid < 0 ? 0 : (valid > V ? V : valid);
-          if (pk + k >= en.k) valid = 0;
-          const T* src = valid ? en.A + (i64)(m0 + r) + (i64)(pk + k) * en.lda : en.A;
-          cp_async_16(as + k * BM + r, src, valid * (int)sizeof(T));
-        }
-      } else {
-        for (int c = tid; c < KS * BM; c += NT) {
-          const int k = c / BM, r = c % BM;
-          const bool ok = r < mrows && pk + k < en.k;
-          const T* src = ok ? en.A + (i64)(m0 + r) + (i64)(pk + k) * en.lda : en.A;
-          cp_async_ca<sizeof(T)>(as + k * BM + r, src, ok ? (int)sizeof(T) : 0);
-        }
-      }
-      for (int c = tid; c < KS * NR; c += NT) {
-        const int k = c / NR, j = c % NR;
-        const bool ok = j < task.n && pk + k < en.k;
-        const T* src = ok ? en.B + (i64)(pk + k) + (i64)j * en.ldb : en.B;
-        cp_async_ca<sizeof(T)>(bs + c, src, ok ? (int)sizeof(T) : 0);
-      }
-      pk += KS;
-      if (pk >= en.k) {
-        pk = 0;
-        pe++;
-        while (pe < task.e1 && ents[pe].k <= 0) pe++;
-      }
-    }
-    cp_async_commit();
-  };
-
-  T acc[2][NR];
-#pragma unroll
-  for (int t = 0; t < 2; t++)
-#pragma unroll
-    for (int j = 0; j < NR; j++) acc[t][j] = T(0);
-
-#pragma unroll
-  for (int s = 0; s < ST - 1; s++) issue(s);
-  // Consumer cursor.
-  int ce = task.e0, ck = 0;
-  while (ce < task.e1 && ents[ce].k <= 0) ce++;
-  int slot = 0;
-  while (ce < task.e1) {
-    const T alpha = ents[ce].alpha;
-    cp_async_wait<ST - 2>();
-    if (alpha != T(1)) {
-      // Scale the B elements this thread copied into the slot.
-      T* bs = Bs + (size_t)slot * KS * NR;
-      for (int c = tid; c < KS * NR; c += NT) bs[c] *= alpha;
-    }
-    __syncthreads();
-    issue((slot + ST - 1) % ST);
-    const T* as = As + (size_t)slot * KS * BM + 2 * tid;
-    const T* bs = Bs + (size_t)slot * KS * NR;
-#pragma unroll
-    for (int k = 0; k < KS; k++) {
-      T a0, a1;
-      if constexpr (sizeof(T) == 8) {
-        const double2 v = *reinterpret_cast<const double2*>(as + k * BM);
-        a0 = v.x;
-        a1 = v.y;
-      } else {
-        const float2 v = *reinterpret_cast<const float2*>(as + k * BM);
-        a0 = v.x;
-        a1 = v.y;
-      }
-#pragma unroll
-      for (int j = 0; j < NR; j++) {
-        const T bj = bs[k * NR + j];
-        acc[0][j] += a0 * bj;
-        acc[1][j] += a1 * bj;
-      }
-    }
-    ck += KS;
-    if (ck >= ents[ce].k) {
-      ck = 0;
-      ce++;
-      while (ce < task.e1 && ents[ce].k <= 0) ce++;
-    }
-    slot = (slot + 1) % ST;
-  }
-  cp_async_wait<0>();
-  // beta C first, so that its loads are all in flight before the first store
-  // (interleaved with the stores each waited for the one before).
-  if (task.beta != T(0))
-#pragma unroll
-    for (int t = 0; t < 2; t++)
-#pragma unroll
-      for (int j = 0; j < NR; j++)
-        if (2 * tid + t < mrows && j < task.n)
-          acc[t][j] = task.beta * task.C[(m0 + 2 * tid + t) + (i64)j * task.ldc] + acc[t][j];
-#pragma unroll
-  for (int t = 0; t < 2; t++) {
-    const int r = 2 * tid + t;
-    if (r >= mrows) continue;
-#pragma unroll
-    for (int j = 0; j < NR; j++) {
-      if (j >= task.n) break;
-      task.C[(m0 + r) + (i64)j * task.ldc] = acc[t][j];
-    }
-  }
-}
-
 // FP64 variant of the streaming apply on the FP64 tensor cores (mma.sync
-// m8n8k4 .f64) for 8 or 16 right-hand sides.  Same ring and cursors as
-// k_stream_nn; each warp owns 32 rows x NR columns as 4 x (NR / 8) m8n8k4
-// accumulators.  A slabs are stored [k][BM + 4] and B slabs [k][NR + 4]
+// m8n8k4 .f64) for 8 or 16 right-hand sides.  Each warp owns 32 rows x NR
+// columns as 4 x (NR / 8) m8n8k4 accumulators.  A slabs are stored [k][BM + 4] and B slabs [k][NR + 4]
 // (doubles): the padding makes the fragment loads of a half-warp (4 k x 4
 // rows or columns) hit 16 distinct bank pairs.  One MMA replaces 8 DFMA
 // instructions per thread, so the apply is no longer issue-bound.
@@ -485,7 +339,9 @@ __global__ void __launch_bounds__(BM, BM == 256 ? 3 : 6)
   }
   cp_async_wait<0>();
   // D fragment: lane holds row lane >> 2, columns 2 (lane & 3) + {0, 1}.
-  if (task.beta != 0.)  // as k_stream_nn
+  // beta C first, so that its loads are all in flight before the first store
+  // (interleaved with the stores each waited for the one before).
+  if (task.beta != 0.)
 #pragma unroll
     for (int i = 0; i < 4; i++)
 #pragma unroll
@@ -741,7 +597,7 @@ __global__ void __launch_bounds__(BM + 32) k_stream_dtma(const GemmTask<double>*
   if (!ok) return;
   // D fragment of 16-row block rb: c[2h + q] is MMA row g8 + 8h (tile row
   // 2 g8 + h of the block), column 2 t4 + q of the column block.
-  if (task.beta != 0.)  // as k_stream_nn
+  if (task.beta != 0.)
 #pragma unroll
     for (int rb = 0; rb < 2; rb++)
 #pragma unroll
@@ -772,8 +628,7 @@ __global__ void __launch_bounds__(BM + 32) k_stream_dtma(const GemmTask<double>*
 
 // FP32 variant of the streaming apply on the tensor cores through warp-level
 // mma.sync m16n8k8 TF32 with the 3-term split (hi*hi + hi*lo + lo*hi, FP32
-// accumulation: FP32 accuracy) for 8 or 16 right-hand sides.  Same ring and
-// cursors as k_stream_nn; each warp owns 32 rows x NR columns as 2 x (NR / 8)
+// accumulation: FP32 accuracy) for 8 or 16 right-hand sides.  Each warp owns 32 rows x NR columns as 2 x (NR / 8)
 // m16n8 accumulators.  A slabs are stored [k][BM + 8] and B slabs [k][NR + 8]
 // (floats) so each fragment load of a warp (8 rows x 4 k) hits 32 distinct
 // banks.  The split happens in registers as fragments are loaded.
@@ -920,7 +775,7 @@ __global__ void __launch_bounds__(BM, BM == 256 ? 3 : 6)
   }
   cp_async_wait<0>();
   // C fragment: c0 (g, 2t), c1 (g, 2t + 1), c2 (g + 8, 2t), c3 (g + 8, 2t + 1).
-  if (task.beta != 0.f)  // as k_stream_nn
+  if (task.beta != 0.f)
 #pragma unroll
     for (int i = 0; i < 2; i++)
 #pragma unroll
@@ -1038,17 +893,6 @@ cudaError_t launch_skinny_nn(int nr, int wide, const GemmTask<T>* d_tasks, const
       return go(k_stream_dmma<16, 128>, stream_dmma_smem<16, 128>(), 128);
     }
   }
-#define H2B_STREAM(NRV)                                                                  \
-  if (nr <= NRV) {                                                                      \
-    if (wide) return go(k_stream_nn<T, NRV, 256>, stream_smem<T, NRV, 256>(), 128);    \
-    return go(k_stream_nn<T, NRV, 128>, stream_smem<T, NRV, 128>(), 64);               \
-  }
-  H2B_STREAM(1)
-  H2B_STREAM(2)
-  H2B_STREAM(4)
-  H2B_STREAM(8)
-  H2B_STREAM(16)
-#undef H2B_STREAM
   return cudaErrorInvalidValue;
 }
 template cudaError_t launch_skinny_nn<double>(int, int, const GemmTask<double>*, const GemmEntry<double>*, const int2*,

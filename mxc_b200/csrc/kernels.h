@@ -136,14 +136,13 @@ template <typename T>
 cudaError_t launch_seg_gemm(int shape, const GemmTask<T>* d_tasks, const GemmEntry<T>* d_ents, const TileRef* d_tiles,
                             int ntiles, cudaStream_t st);
 int gemm_tile_m(int shape);
-// Plans whose entries all use A and B as stored and whose outputs have at
-// most 16 columns: A streamed from HBM through a shared-memory ring, one CTA
-// per skinny_rows_per_cta(wide) rows of a task (tile = {task, row block});
-// wide = 0 for tasks of at most 128 rows, 1 otherwise.  FP64 plans with 5-16
-// columns given bulk_err (a device int) run the warp-specialised bulk-copy
-// kernel, which wants every A column start 16-byte aligned for full speed
-// and sets *bulk_err when one of its mbarrier waits expires; without
-// bulk_err they run the cp.async ring.
+// Plans whose entries all use A and B as stored and whose outputs have 5 to 16
+// columns: A streamed from HBM through a shared-memory ring, one CTA per
+// skinny_rows_per_cta(wide) rows of a task (tile = {task, row block}); wide = 0
+// for tasks of at most 128 rows, 1 otherwise.  FP64 plans given bulk_err (a
+// device int) run the warp-specialised bulk-copy kernel, which wants every A
+// column start 16-byte aligned for full speed and sets *bulk_err when one of
+// its mbarrier waits expires; without bulk_err they run the cp.async ring.
 template <typename T>
 cudaError_t launch_skinny_nn(int nr, int wide, const GemmTask<T>* d_tasks, const GemmEntry<T>* d_ents,
                              const int2* d_tiles, int ntiles, cudaStream_t st, int* bulk_err = nullptr);
@@ -233,8 +232,7 @@ struct BfEntry {
 cudaError_t launch_apply_bf16(int nr, int rl, const GemmTask<float>* d_tasks, const BfEntry* d_ents,
                               const int2* d_tiles, int ntiles, cudaStream_t st);
 cudaError_t launch_bf16_pack(const BfPackTask* d_tasks, int ntasks, cudaStream_t st);
-// 5-16 right-hand sides run on the BF16 tensor cores (k_stream_bf16_mma),
-// 1-4 on the FMA pipe.
+// 5-16 right-hand sides on the BF16 tensor cores (k_stream_bf16_mma).
 cudaError_t launch_stream_bf16(int nr, const GemmTask<float>* d_tasks, const BfEntry* d_ents, const int2* d_tiles,
                                int ntiles, cudaStream_t st);
 int bf16_rows_per_cta();

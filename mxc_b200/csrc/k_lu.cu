@@ -9,11 +9,16 @@ namespace h2b {
 
 // Factorization, one CTA per box: pivot = first row of largest magnitude in
 // column k among rows k..n-1, the column below it divided by it, rank-1 update
-// of the trailing block.  Blocked by panels of NB columns, but every element
-// takes its updates one multiply-add at a time in the order of k, so the
-// factor is bit for bit that of the unblocked elimination -- which matters for
-// the ill-conditioned reference configuration, whose substitution moves by
-// tens of percent with the rounding order.
+// of the trailing block.  Blocked by panels of NB columns.  In FP64, and in
+// FP32 in shared memory, every element takes its updates one multiply-add at a
+// time in the order of k, so the factor is bit for bit that of the unblocked
+// elimination -- which matters for the ill-conditioned reference
+// configuration, whose substitution moves by tens of percent with the rounding
+// order.  FP32 in global scratch (SUMS) subtracts a panel's NB products from an
+// element of the trailing block as one sum, which keeps the rounding error of a
+// diagonally dominant block at 2.5e-7 of it from 256 to 900 rows (one at a time:
+// 1.9e-6 to 6.5e-6, so a substitution's root block moved by 2e-6 and the result
+// of its BF16 copy by 1e-4).
 //
 // Bound: the chain of pivots.  A panel's rows live in registers (RPT rows of
 // NB columns per thread) and a pivot costs two barriers: the warps' candidates
@@ -57,6 +62,7 @@ __device__ __forceinline__ void lu_warp_best(unsigned long long& key, int& row) 
 template <typename T, int NT, int NB, int RPT, bool SMEM>
 __global__ void __launch_bounds__(NT) k_lu_factor(const LuSolveTask<T>* __restrict__ tasks) {
   constexpr int NW = NT / 32;
+  constexpr bool SUMS = !SMEM && sizeof(T) == 4;
   const LuSolveTask<T> t = tasks[blockIdx.x];
   const int n = t.n;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
@@ -239,7 +245,8 @@ __global__ void __launch_bounds__(NT) k_lu_factor(const LuSolveTask<T>* __restri
         if (i < kb) ac[i] = u[i];
     }
     __syncthreads();
-    // Trailing block, LU_TT x LU_TT tiles, updates in the order of k.
+    // Trailing block, LU_TT x LU_TT tiles, updates in the order of k.  acc: the
+    // element itself, or (SUMS) minus the panel's products.
     constexpr int GX = 16, GY = NT / GX, TY = LU_TT / GY, TX = LU_TT / GX;
     const int tx = tid % GX, ty = tid / GX;
     for (int tc = j0; tc < n; tc += LU_TT)
@@ -250,7 +257,7 @@ __global__ void __launch_bounds__(NT) k_lu_factor(const LuSolveTask<T>* __restri
 #pragma unroll
           for (int u = 0; u < TX; u++) {
             const int r = tr + tx + GX * u, c = tc + ty + GY * v;
-            acc[u][v] = (r < n && c < n) ? a[r + (size_t)c * ld] : T(0);
+            acc[u][v] = (!SUMS && r < n && c < n) ? a[r + (size_t)c * ld] : T(0);
           }
         for (int e = tid; e < LU_TT * NB; e += NT) {
           const int rr = e % LU_TT, i = e / LU_TT;
@@ -274,6 +281,14 @@ __global__ void __launch_bounds__(NT) k_lu_factor(const LuSolveTask<T>* __restri
 #pragma unroll
             for (int v = 0; v < TY; v++) acc[u][v] -= lv[u] * uv[v];
         }
+        if (SUMS)
+#pragma unroll
+          for (int v = 0; v < TY; v++)
+#pragma unroll
+            for (int u = 0; u < TX; u++) {
+              const int r = tr + tx + GX * u, c = tc + ty + GY * v;
+              if (r < n && c < n) acc[u][v] += a[r + (size_t)c * ld];
+            }
 #pragma unroll
         for (int v = 0; v < TY; v++)
 #pragma unroll
@@ -425,8 +440,9 @@ cudaError_t launch_lu_solve(const LuSolveTask<T>* d_tasks, int ntasks, int maxn,
   cudaError_t e;
   if (in_smem) e = go(k_lu_factor<T, 256, 32, 1, true>, 256);
   else if (maxn <= 512) e = go(k_lu_factor<T, 512, 32, 1, false>, 512);
-  else if (maxn <= 1024) e = go(k_lu_factor<T, 512, 16, 2, false>, 512);
-  else e = go(k_lu_factor<T, 512, 8, 4, false>, 512);
+  // Beyond, as many columns as the registers hold (64 a thread of 512).
+  else if (maxn <= 1024) e = go(k_lu_factor<T, 512, sizeof(T) == 4 ? 32 : 16, 2, false>, 512);
+  else e = go(k_lu_factor<T, 512, sizeof(T) == 4 ? 16 : 8, 4, false>, 512);
   if (e != cudaSuccess || maxm <= 0) return e;
   note_launch();
   k_lu_trsm<T><<<dim3(ntasks, (maxm + LU_CT - 1) / LU_CT), LU_CT, 0, st>>>(d_tasks);

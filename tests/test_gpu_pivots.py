@@ -31,6 +31,57 @@ def test_single_box_solve_is_backward_stable(handle, n, precision):
     assert np.linalg.norm(K @ x - rhs) < bound
 
 
+def _fma32(c, x, y):
+    """c - x y rounded once to float32 (twice where the double lies on a tie: about 1 in 2^29)."""
+    return (c.astype(float) - x.astype(float) * y.astype(float)).astype(np.float32)
+
+
+def _inverse_fp32(K, panel):
+    """The inverse by a float32 LU with partial pivoting that subtracts `panel` products from an element of
+    the trailing block as one sum, and the solve's order of operations (32 rows at a time)."""
+    a, n = K.astype(np.float32), len(K)
+    p = np.arange(n)
+    for k0 in range(0, n, panel):
+        j0 = min(k0 + panel, n)
+        for k in range(k0, j0):
+            q = k + int(np.argmax(abs(a[k:, k])))
+            a[[k, q]], p[[k, q]] = a[[q, k]], p[[q, k]]
+            a[k + 1:, k] /= a[k, k]
+            a[k + 1:, k + 1:j0] = _fma32(a[k + 1:, k + 1:j0], a[k + 1:, k:k + 1], a[k:k + 1, k + 1:j0])
+        for i in range(k0, j0):
+            a[i + 1:j0, j0:] = _fma32(a[i + 1:j0, j0:], a[i + 1:j0, i:i + 1], a[i:i + 1, j0:])
+        s = np.zeros_like(a[j0:, j0:])
+        for i in range(k0, j0):
+            s = _fma32(s, a[j0:, i:i + 1], a[i:i + 1, j0:])
+        a[j0:, j0:] += s
+    X = np.eye(n, dtype=np.float32)[p]
+    for j in range(n):
+        X[j + 1:] = _fma32(X[j + 1:], a[j + 1:, j:j + 1], X[j:j + 1])
+    for b0 in range((n - 1) // 32 * 32, -1, -32):
+        e = min(b0 + 32, n)
+        for j in range(e, n):
+            X[b0:e] = _fma32(X[b0:e], a[b0:e, j:j + 1], X[j:j + 1])
+        for j in range(e - 1, b0 - 1, -1):
+            X[j] /= a[j, j]
+            X[b0:j] = _fma32(X[b0:j], a[b0:j, j:j + 1], X[j:j + 1])
+    return X
+
+
+@pytest.mark.parametrize("n", [257, 320, 513, 700])
+def test_fp32_factor_in_scratch_sums_by_panels(handle, n):
+    """FP32 blocks beyond shared memory: the inverse is that of an LU whose
+    trailing updates are sums of 32 products, operation for operation (the
+    margin is for a double rounding of the restatement; updates one product at
+    a time move it by 1e-6 and more)."""
+    b = np.random.default_rng(n).random((n, 3))
+    M = m.H2MatrixSolver(handle, m.Laplace3D(1e-4), 0.0, 8, 0, m.build_tree(b, 0), 2.0, b, precision=m.FP32)
+    K = M.export(0, m._lib.EXPORT_A).reshape(n, n).T
+    assert M.factorizeM() == [0]
+    got = M.export(0, m._lib.EXPORT_R).reshape(n, n)
+    ref = _inverse_fp32(K, 32)
+    assert np.linalg.norm(got - ref) < 1e-7 * np.linalg.norm(ref)
+
+
 @pytest.mark.parametrize("box", [20, 33, 156, 157, 256, 257, 312, 480, 513, 650, 769])
 @pytest.mark.parametrize("eps", [1e-3, 1e-9])
 def test_operator_box_sizes(handle, box, eps):

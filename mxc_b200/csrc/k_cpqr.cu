@@ -106,7 +106,9 @@ __global__ void __launch_bounds__(CPQR_NT) k_cpqr_cluster(const i64* __restrict_
       pos[l] = c0 + l;
     }
   }
-  __syncthreads();
+  // Of the whole cluster: the first candidates go to the other CTAs' shared
+  // memory, which may be written only once those CTAs are known to run.
+  cl.sync();
   int steps = K < M ? K : M;
   const double eps = (sizeof(T) == 8) ? DBL_EPSILON : (double)FLT_EPSILON;
   const double downdate_thr = sqrt(eps);

@@ -107,6 +107,32 @@ def test_operator_box_sizes(handle, box, eps):
     assert np.linalg.norm(y - d) < 10 * eps * np.linalg.norm(d)
 
 
+def test_operator_boxes_smaller_than_their_cluster(handle):
+    """A level of boxes of 3 to 256 bodies runs its pivoted QRs on clusters
+    sized for the largest: CTAs of the small ones start late and own no column.
+    The product is within ten times the threshold of the dense one, the points
+    stay a permutation and repeated builds give the same bits."""
+    rng = np.random.default_rng(0)
+    b = np.concatenate([0.1 * rng.random((900, 3)), rng.random((60, 3))])
+    t = m.build_tree(b, 4, 3, 256)
+    k, eps, first = m.Laplace3D(1e-2), 1e-9, None
+    x = np.random.default_rng(2).random(len(b))
+    for _ in range(5):
+        A = m.H2MatrixSolver(handle, k, eps, 100, 0, t, 1.0, b)
+        dims, ranks = A.level_dims(4)
+        assert dims.min() == 3 and dims.max() == 256 and np.all(ranks <= dims)
+        S = A.export(4, m._lib.EXPORT_S).reshape(-1, 3)
+        assert np.array_equal(S[np.lexsort(S.T)], b[np.lexsort(b.T)])
+        y = x.copy()
+        A.matVecMul(y)
+        A.close()
+        if first is None:
+            d = m.dense_matvec(handle, k, b, x)
+            assert np.linalg.norm(y - d) < 10 * eps * np.linalg.norm(d)
+            first = y, S
+        assert np.array_equal(y, first[0]) and np.array_equal(S, first[1])
+
+
 @pytest.mark.parametrize("box,seed", [(20, 1), (64, 2), (130, 3), (321, 4)])
 @pytest.mark.parametrize("precision", [m.FP64, m.FP32])
 def test_sketched_operator_box_sizes(box, seed, precision):

@@ -520,7 +520,7 @@ struct GemmPlan {
       }
       d_rtiles.put(packed, rt[0]);
       d_rtiles_w.put(packed, rt[1]);
-      tkey = tune_key(name, (int)sizeof(T), nr, (double)tasks.size(), rows, elems);
+      tkey = tune_key(name, (int)sizeof(T), nr, (double)tasks.size(), rows, elems) + "/rows";  // variants of its own
     }
     if (skinny_nn && !by_rows) split_tasks();
     if (skinny_nn && !by_rows) {

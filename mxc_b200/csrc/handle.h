@@ -44,9 +44,10 @@ struct h2dev_handle_s {
   bool precond_bf16 = false;
   bool graph_solve = false;
   // Autotuner (H2DEV_OPT_AUTOTUNE): the launch variant chosen for each plan
-  // shape bucket (key: plan name, element size, right-hand sides and
-  // log2-bucketed task / row / element counts) and the device times each
-  // variant took when it was measured.
+  // shape bucket (key: plan name, element size, right-hand sides,
+  // log2-bucketed task / row / element counts, and the kernel where a plan's
+  // sums decide it) and the device times each variant took when it was
+  // measured.
   bool autotune = true;
   struct TuneRec {
     int choice;

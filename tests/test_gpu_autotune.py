@@ -58,3 +58,22 @@ def test_autotuned_applies_equal_default_applies(mf):
         s.close()
     h1.close()
     h2.close()
+
+
+def test_plans_of_two_kernels_are_tuned_apart():
+    """Two plans of one size bucket, the first of 200 row tiles of 128 (by
+    rows: two tilings), the second of 400 (the ring: three): each is measured."""
+    import ctypes as C
+
+    import torch
+
+    h = m.Handle(0)
+    A, B, Y = (torch.rand(200 * n, dtype=torch.float32, device="cuda") for n in (129 * 64, 64 * 16, 129 * 16))
+    torch.cuda.synchronize()
+    for rows in (128, 129):
+        m._lib.check(m._lib.lib().h2dev_batched_gemm_device(
+            h.h, m.FP32, 200, 1, rows, 16, 64, 0, 0, 1.0, C.c_void_p(A.data_ptr()), rows, rows * 64,
+            C.c_void_p(B.data_ptr()), 64, 64 * 16, 0.0, C.c_void_p(Y.data_ptr()), rows, rows * 16), "gemm")
+    h.synchronize()
+    assert [len(ms) for _, _, ms in h.autotune_report()] == [2, 3]
+    h.close()

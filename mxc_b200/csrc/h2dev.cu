@@ -465,7 +465,7 @@ struct GemmPlan {
   // repeating one leaves the same result, so tuning runs are harmless.
   bool idempotent = false;
   // By-rows plans (k_apply): d_rtiles / d_rtiles_w are the tilings of 1 and 2
-  // rows per lane, the autotuner's two variants.
+  // rows per lane (two where apply_max_rl allows them: the autotuner's variants).
   bool by_rows = false;
   // FP64 streaming plans whose A columns all start on 16-byte boundaries run
   // the bulk-copy kernel.
@@ -513,7 +513,7 @@ struct GemmPlan {
         const auto& t = tasks[ti];
         if (t.m <= 0 || t.n <= 0) continue;
         if (t.e0 == t.e1 && t.beta == T(1)) continue;
-        for (int v = 0; v < 2; v++)
+        for (int v = 0; v < apply_max_rl(sizeof(T), nr); v++)
           for (int a = 0; a < t.m; a += apply_rows_per_cta(v + 1)) rt[v].push_back(make_int2(ti, a / apply_rows_per_cta(v + 1)));
         rows += t.m;
         for (int e = t.e0; e < t.e1; e++) elems += (double)t.m * ents[e].k;
@@ -698,8 +698,9 @@ struct GemmPlan {
 
   void run_skinny(int v, cudaStream_t st) const {
     if (by_rows) {
-      const DView<int2>& t = v == 0 ? d_rtiles_w : d_rtiles;
-      ck(launch_apply<T>(nr, v == 0 ? 2 : 1, d_tasks.p, d_ents.p, t.p, (int)t.n, st), "apply");
+      const int rl = v == 0 ? apply_max_rl(sizeof(T), nr) : 1;
+      const DView<int2>& t = rl == 2 ? d_rtiles_w : d_rtiles;
+      ck(launch_apply<T>(nr, rl, d_tasks.p, d_ents.p, t.p, (int)t.n, st), "apply");
       return;
     }
     const DView<int2>& w = v == 0 ? d_rtiles_w : d_alt_w;
@@ -718,7 +719,7 @@ struct GemmPlan {
       variant = 0;
       return;
     }
-    const int v = tuned_variant(tkey, by_rows ? 2 : 3, st, [&](int x) { run_skinny(x, st); });
+    const int v = tuned_variant(tkey, by_rows ? apply_max_rl(sizeof(T), nr) : 3, st, [&](int x) { run_skinny(x, st); });
     if (!stream_capturing(st)) variant = v;
   }
 

@@ -218,15 +218,25 @@ static cudaError_t apply_go(const GemmTask<T>* tasks, const ENT* ents, const int
 }
 
 int apply_rows_per_cta(int rl) { return 32 * rl; }
+// Rows per lane up to which k_apply is built.  FP64 with at most 8 columns has
+// one: two rows of a chunk in use and two on their way fill the 128 registers of
+// a thread at two CTAs per SM and spilled (substitution of 65,536 bodies, FP64: 4
+// columns 1,302 us with two rows, 981 with one; 8 columns of 32,768: 845, 740).
+// With 16 two rows are the faster form (32,768: 856, 899), as in FP32 (65,536, 1
+// column: 650, 785).
+int apply_max_rl(size_t elem, int nr) { return elem == 8 && nr <= 8 ? 1 : 2; }
 
 template <typename AT, typename T, typename ENT>
 static cudaError_t apply_any(int nr, int rl, const GemmTask<T>* tasks, const ENT* ents, const int2* tiles, int ntiles,
                              cudaStream_t st) {
   if (ntiles == 0) return cudaSuccess;
 #define H2B_APPLY(N)                                                                             \
-  if (nr <= N)                                                                                   \
-    return rl == 1 ? apply_go<AT, T, ENT, N, 1, 8>(tasks, ents, tiles, ntiles, st)               \
-                   : apply_go<AT, T, ENT, N, 2, 8>(tasks, ents, tiles, ntiles, st);
+  if (nr <= N) {                                                                                 \
+    if constexpr (sizeof(T) == 4 || N > 8) {                                                     \
+      if (rl == 2) return apply_go<AT, T, ENT, N, 2, 8>(tasks, ents, tiles, ntiles, st);         \
+    }                                                                                            \
+    if (rl == 1) return apply_go<AT, T, ENT, N, 1, 8>(tasks, ents, tiles, ntiles, st);           \
+  }
   H2B_APPLY(1)
   H2B_APPLY(2)
   H2B_APPLY(4)

@@ -148,11 +148,12 @@ cudaError_t launch_skinny_nn(int nr, int wide, const GemmTask<T>* d_tasks, const
                              const int2* d_tiles, int ntiles, cudaStream_t st, int* bulk_err = nullptr);
 int skinny_rows_per_cta(int wide);
 // The same products by rows (k_apply.cu): one CTA per apply_rows_per_cta(rl)
-// rows of a task, rl = 1 or 2; both give the same bits.
+// rows of a task, rl = 1 to apply_max_rl; both give the same bits.
 template <typename T>
 cudaError_t launch_apply(int nr, int rl, const GemmTask<T>* d_tasks, const GemmEntry<T>* d_ents, const int2* d_tiles,
                          int ntiles, cudaStream_t st);
 int apply_rows_per_cta(int rl);
+int apply_max_rl(size_t elem, int nr);
 // Reduction of a split task: dst (m x n, ld ldd) = beta dst + sum of `parts`
 // consecutive m x n partial results at src.
 template <typename T>

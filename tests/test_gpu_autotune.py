@@ -77,3 +77,25 @@ def test_plans_of_two_kernels_are_tuned_apart():
     h.synchronize()
     assert [len(ms) for _, _, ms in h.autotune_report()] == [2, 3]
     h.close()
+
+
+def test_fp64_plans_by_rows_have_one_tiling_up_to_8_columns():
+    """One row per lane: there is nothing to measure for FP64 plans of at most
+    8 columns (the two-row form spilled and was 10 to 50% slower), two tilings
+    beyond, and in FP32."""
+    import ctypes as C
+
+    import torch
+
+    h = m.Handle(0)
+    A, B, Y = (torch.rand(4 * n, dtype=torch.float64, device="cuda") for n in (128 * 64, 64 * 16, 128 * 16))
+    torch.cuda.synchronize()
+    seen = []
+    for precision, cols in ((m.FP64, 1), (m.FP64, 4), (m.FP64, 8), (m.FP64, 9), (m.FP32, 4)):
+        m._lib.check(m._lib.lib().h2dev_batched_gemm_device(
+            h.h, precision, 4, 1, 128, cols, 64, 0, 0, 1.0, C.c_void_p(A.data_ptr()), 128, 128 * 64,
+            C.c_void_p(B.data_ptr()), 64, 64 * cols, 0.0, C.c_void_p(Y.data_ptr()), 128, 128 * cols), "gemm")
+        seen.append([len(ms) for _, _, ms in h.autotune_report()])
+    assert seen == [[], [], [], [2], [2, 2]]
+    h.synchronize()
+    h.close()

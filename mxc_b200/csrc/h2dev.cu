@@ -992,8 +992,8 @@ struct Level {
   DVec<T> Q, R, A, C;
   std::vector<i64> na_off, na_ld;  // destination of each near block's ss part in the parent A
   // factorization results
-  DVec<T> B, invT;
-  std::vector<i64> boff, ioff;
+  DVec<T> B;
+  std::vector<i64> boff;
   DVec<int> ipiv, info;
   int info_count = 0;
   // Transposed copies for the multi-RHS applies, so every apply streams
@@ -2103,19 +2103,14 @@ class Solver : public SolverBase {
     DVec<T> T1;
     T1.alloc(lv.qoff[nodes]);
     lv.boff.assign(nodes + 1, 0);
-    lv.ioff.assign(nodes + 1, 0);
     std::vector<i64> poff(nodes + 1, 0);
     for (i64 i = 0; i < nodes; i++) {
       i64 Mr = D[i] - Rk[i];
       lv.boff[i + 1] = lv.boff[i] + Mr * D[i];
-      lv.ioff[i + 1] = lv.ioff[i] + Mr * Mr;
       poff[i + 1] = poff[i] + Mr;
     }
     lv.B.alloc(std::max<i64>(1, lv.boff[nodes]));
-    // The factors of the redundant blocks (released at the end of the level),
-    // their pivots and row orders.
-    lv.invT.alloc(std::max<i64>(1, lv.ioff[nodes]));
-    lv.ipiv.alloc(std::max<i64>(1, 2 * poff[nodes]));
+    lv.ipiv.alloc(std::max<i64>(1, 2 * poff[nodes]));  // pivots and row orders
     lv.info.alloc(nodes);
     lv.info.zero(st());
     T* A = lv.A.p;
@@ -2157,7 +2152,7 @@ class Solver : public SolverBase {
       t.m = M;
       t.X = V + lv.qoff[i] + (i64)Ms * M;
       t.ldx = M;
-      t.work = lv.invT.p + lv.ioff[i];
+      t.work = lv.B.p + lv.boff[i];  // the factor, until step 8 writes B
       t.ipiv = lv.ipiv.p + poff[i];
       t.prow = lv.ipiv.p + poff[nodes] + poff[i];
       t.info = lv.info.p + i;
@@ -2312,7 +2307,6 @@ class Solver : public SolverBase {
       s10.run(st());
       s11b.run(st());
     }
-    lv.invT.release();
   }
 
   void copy_next(i64 l) {

@@ -31,6 +31,25 @@ def test_single_box_solve_is_backward_stable(handle, n, precision):
     assert np.linalg.norm(K @ x - rhs) < bound
 
 
+@pytest.mark.parametrize("precision", [m.FP64, m.FP32])
+@pytest.mark.parametrize("n", [128, 1024])
+def test_factorization_memory(n, precision):
+    """The LU factors of the redundant blocks need no memory of their own: a
+    box takes A U and B beside what the solver holds (powers of two, the size
+    classes of the handle's cache), and the plans."""
+    b = np.random.default_rng(n).random((n, 3))
+    h = m.Handle(0)
+    M = m.H2MatrixSolver(h, m.Laplace3D(1e-2), 0.0, 8, 0, m.build_tree(b, 0), 2.0, b, precision=precision)
+    h.synchronize()
+    live = h.memory()[0]
+    h.memory_peak(reset=True)
+    M.factorizeM()
+    block = n * n * (8 if precision == m.FP64 else 4)
+    assert h.memory_peak() - live <= 2 * block + 32768
+    M.close()
+    h.close()
+
+
 def _fma32(c, x, y):
     """c - x y rounded once to float32 (twice where the double lies on a tie: about 1 in 2^29)."""
     return (c.astype(float) - x.astype(float) * y.astype(float)).astype(np.float32)

@@ -1463,28 +1463,25 @@ class Solver : public SolverBase {
               if (S > M) sfl += 2. * (double)M * (double)M * (double)S;
               longest = std::max(longest, S);
             }
-            // The parts' sums take at most 512 MB beside the level's own blocks.
+            // More than one part: their sums take at most 512 MB beside the
+            // level's own blocks.
             int parts = sketch_parts((i64)tiles.size(), tm, longest);
             while (parts > 1 && (i64)parts * lv.qoff[nodes] > ((i64)1 << 26)) parts--;
-            const size_t ntl = tiles.size();
-            for (int p = 1; p < parts; p++)
-              for (size_t z = 0; z < ntl; z++) tiles.push_back(make_int4(tiles[z].x, tiles[z].y, tiles[z].z, p));
             DVec<i64> d_roff, d_rstart, d_rend;
             DVec<int4> d_tiles;
-            DVec<double> Y;
             d_roff.upload(roff);
             d_rstart.upload(rstart);
             d_rend.upload(rend);
+            DVec<double> Y;
+            if (parts > 1) Y.alloc((size_t)parts * lv.qoff[nodes]);
+            const size_t ntl = tiles.size();
+            for (int p = 1; p < parts; p++)
+              for (size_t z = 0; z < ntl; z++) tiles.push_back(make_int4(tiles[z].x, tiles[z].y, tiles[z].z, p));
             d_tiles.upload(tiles);
-            double* y = reinterpret_cast<double*>(Rws.p);
-            if (parts > 1 || !std::is_same<T, double>::value) {
-              Y.alloc((size_t)parts * lv.qoff[nodes]);
-              y = Y.p;
-            }
             Prof pf("sketch", sfl, 24. * (double)soff[nodes]);
             ck(launch_sketch<T>(kp, bodies.p, lv.pts.p, lv.d_xoff.p, lv.d_dims.p, lv.d_qoff.p, d_roff.p, d_rstart.p,
-                                d_rend.p, d_tiles.p, (int)tiles.size(), tm, parts, lv.qoff[nodes], y, Rws.p,
-                                (int)nodes, st()),
+                                d_rend.p, d_tiles.p, (int)tiles.size(), tm, parts, lv.qoff[nodes],
+                                parts > 1 ? Y.p : reinterpret_cast<double*>(Rws.p), Rws.p, (int)nodes, st()),
                "sketch");
           } else {
             Prof pf("sample_tsqr", fl, (double)sidx.size() * 28.);

@@ -91,7 +91,7 @@ __global__ void __launch_bounds__(64 * WM + 32, sketch_ctas(WM))
     k_sketch(KernelParams kp_in, const double* __restrict__ bodies, const double* __restrict__ pts,
              const i64* __restrict__ xoff, const i64* __restrict__ dims, const i64* __restrict__ qoff,
              const i64* __restrict__ roff, const i64* __restrict__ rstart, const i64* __restrict__ rend,
-             const int4* __restrict__ tiles, int parts, i64 pstride, double* __restrict__ Y) {
+             const int4* __restrict__ tiles, int parts, i64 pstride, double* __restrict__ Y, float* __restrict__ F) {
   constexpr int TM = 32 * WM, NMMA = 64 * WM;  // threads that multiply
   __shared__ __align__(16) double xf[2][SK_TN * SK_CS];
   __shared__ double fc[2][SK_KS * 3];
@@ -107,7 +107,7 @@ __global__ void __launch_bounds__(64 * WM + 32, sketch_ctas(WM))
   const int a0 = tl.y * TM, c0 = tl.z * SK_TN;
   const i64 r0 = roff[box], r1 = roff[box + 1];
   const i64 S = r1 > r0 ? rend[r1 - 1] : 0;
-  double* W = Y + (i64)tl.w * pstride + qoff[box];
+  double* W = Y + (i64)tl.w * pstride + qoff[box];  // F (FP32 bases in one piece): stored there instead
   const double* X = pts + 3 * xoff[box];
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   if (M == 0 || S == 0) return;
@@ -119,8 +119,12 @@ __global__ void __launch_bounds__(64 * WM + 32, sketch_ctas(WM))
       const int a = a0 + e / SK_TN, c = c0 + e % SK_TN;
       if ((i64)a >= S || c >= M) continue;
       const i64 body = sk_body(a, r0, r0, rstart, rend);
-      W[(i64)a * M + c] = kernel_fast_pair(kp, bodies[3 * body], bodies[3 * body + 1], bodies[3 * body + 2], X[3 * c],
-                                           X[3 * c + 1], X[3 * c + 2]);
+      const double v = kernel_fast_pair(kp, bodies[3 * body], bodies[3 * body + 1], bodies[3 * body + 2], X[3 * c],
+                                        X[3 * c + 1], X[3 * c + 2]);
+      if (F)
+        F[qoff[box] + (i64)a * M + c] = (float)v;
+      else
+        W[(i64)a * M + c] = v;
     }
     return;
   }
@@ -228,7 +232,11 @@ __global__ void __launch_bounds__(64 * WM + 32, sketch_ctas(WM))
 #pragma unroll
       for (int h = 0; h < 2; h++) {
         const int col = c0 + wn * 32 + j * 8 + 2 * (lane & 3) + h;
-        if (a < M && col < M) W[(i64)a * M + col] = acc[i][j][h];
+        if (a >= M || col >= M) continue;
+        if (F)
+          F[qoff[box] + (i64)a * M + col] = (float)acc[i][j][h];
+        else
+          W[(i64)a * M + col] = acc[i][j][h];
       }
   }
 }
@@ -279,10 +287,12 @@ cudaError_t launch_sketch(const KernelParams& kp, const double* bodies, const do
                           const int4* d_tiles, int ntiles, int tile_rows, int parts, i64 pstride, double* Y, T* Rws,
                           int nboxes, cudaStream_t st) {
   if (ntiles == 0) return cudaSuccess;
+  float* f32 = nullptr;
+  if constexpr (std::is_same<T, float>::value) f32 = parts == 1 ? Rws : nullptr;
   auto go = [&](auto kern, int wm) {
     note_launch();
     kern<<<ntiles, 64 * wm + 32, 0, st>>>(kp, bodies, pts, xoff, dims, qoff, roff, rstart, rend, d_tiles, parts,
-                                          pstride, Y);
+                                          pstride, Y, f32);
     return cudaGetLastError();
   };
   cudaError_t e = cudaErrorInvalidValue;
@@ -292,7 +302,7 @@ cudaError_t launch_sketch(const KernelParams& kp, const double* bodies, const do
     H2B_SK(1) H2B_SK(2) H2B_SK(3) H2B_SK(4) H2B_SK(5) H2B_SK(6) H2B_SK(7) H2B_SK(8) H2B_SK(9) H2B_SK(10)
 #undef H2B_SK
   }
-  if (e != cudaSuccess || (std::is_same<T, double>::value && parts == 1)) return e;
+  if (e != cudaSuccess || parts == 1) return e;
   note_launch();
   k_sketch_sum<T><<<dim3(nboxes, 16), 256, 0, st>>>(dims, qoff, roff, rend, Y, parts, pstride, Rws);
   return cudaGetLastError();

@@ -35,7 +35,7 @@ cudaError_t launch_sample_tsqr(const KernelParams& kp, const double* bodies, con
 // over every far body (ranges roff[box]..roff[box+1]-1 of rstart / rend), or
 // the first S rows = XF when S <= M.  tiles: {box, row tile, column tile, part}
 // for every part of 0..parts-1; Y: the parts' sums, pstride doubles apart
-// (FP64 with one part: Rws itself).
+// (unused with one part: stored to Rws).
 template <typename T>
 cudaError_t launch_sketch(const KernelParams& kp, const double* bodies, const double* pts, const i64* xoff,
                           const i64* dims, const i64* qoff, const i64* roff, const i64* rstart, const i64* rend,

@@ -134,3 +134,26 @@ def test_sketch_near_levels_plus_samples_matches_oracle(handle):
     # Cheaper than the whole far field, and less accurate (at 16,384 bodies
     # about 7x the full sketch's error, still well inside the threshold).
     assert rel(yf, yd) < 1e-12 and rel(y, yd) < 1e-11
+
+
+def _sketched(h, n, levels, theta, eps, precision, bodies, samples):
+    t = m.build_tree(bodies, levels)
+    h.set_option(m._lib.OPT_SAMPLING, m._lib.SAMPLING_SKETCH)
+    return m.H2MatrixSolver(h, m.Laplace3D(1e-2), eps, 100, 0, t, theta, bodies, samples=samples, precision=precision)
+
+
+def test_fp32_sketch_in_one_part_needs_no_copy():
+    """2,048 boxes of 32 bodies on a line fill the chip with one part of their
+    far lists, whose sketch is stored in FP32 at once: at the leaves an operator
+    holds its near blocks, the bases' three arrays, the bodies twice, lists and
+    couplings (17 MB; an FP64 copy of the sketch would be as much again)."""
+    n = 65536
+    b = np.zeros((n, 3))
+    b[:, 0] = np.random.default_rng(0).random(n)
+    h = m.Handle(0)
+    A = _sketched(h, n, 11, 1.0, 1e-4, m.FP32, b, 500)
+    near = m.pair_csr("N", m.build_tree(b.copy(), 11), 1.0)[0]
+    blocks = int(near[-1] - near[2047])
+    assert h.memory_peak() < 4 * 1024 * (blocks + 3 * 2048) + 48 * n + 24e6
+    A.close()
+    h.close()

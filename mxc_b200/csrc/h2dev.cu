@@ -1464,7 +1464,8 @@ class Solver : public SolverBase {
               longest = std::max(longest, S);
             }
             // More than one part: their sums take at most 512 MB beside the
-            // level's own blocks.
+            // level's own blocks, and where that does not fit the far list is
+            // taken in one piece.
             int parts = sketch_parts((i64)tiles.size(), tm, longest);
             while (parts > 1 && (i64)parts * lv.qoff[nodes] > ((i64)1 << 26)) parts--;
             DVec<i64> d_roff, d_rstart, d_rend;
@@ -1473,7 +1474,12 @@ class Solver : public SolverBase {
             d_rstart.upload(rstart);
             d_rend.upload(rend);
             DVec<double> Y;
-            if (parts > 1) Y.alloc((size_t)parts * lv.qoff[nodes]);
+            try {
+              if (parts > 1) Y.alloc((size_t)parts * lv.qoff[nodes]);
+            } catch (const H2Error& x) {
+              if (x.code != H2DEV_ERR_OOM) throw;
+              parts = 1;
+            }
             const size_t ntl = tiles.size();
             for (int p = 1; p < parts; p++)
               for (size_t z = 0; z < ntl; z++) tiles.push_back(make_int4(tiles[z].x, tiles[z].y, tiles[z].z, p));

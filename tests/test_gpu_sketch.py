@@ -157,3 +157,32 @@ def test_fp32_sketch_in_one_part_needs_no_copy():
     assert h.memory_peak() < 4 * 1024 * (blocks + 3 * 2048) + 48 * n + 24e6
     A.close()
     h.close()
+
+
+def test_sketch_in_parts_falls_back_to_one_part():
+    """Where the sums of the parts do not fit the card (8 boxes of 640: 98 MB
+    beside 243), the far lists are taken in one piece: the operator is built
+    in 285 MB and is as accurate."""
+    import torch
+
+    n = 5120
+    b = np.random.default_rng(3).random((n, 3))
+    x = np.random.default_rng(2).random(n)
+    h = m.Handle(0)
+    A = _sketched(h, n, 3, 1.0, 1e-8, m.FP64, b, 4000)  # loads the kernels
+    A.close()
+    h.trim()
+    torch.zeros(1, device="cuda")
+    free = torch.cuda.mem_get_info()[0]
+    fill = torch.empty(free - 285_000_000, dtype=torch.uint8, device="cuda")
+    try:
+        A = _sketched(h, n, 3, 1.0, 1e-8, m.FP64, b, 4000)
+    finally:
+        del fill
+        torch.cuda.empty_cache()
+    d = m.dense_matvec(h, m.Laplace3D(1e-2), b, x)
+    y = x.copy()
+    A.matVecMul(y)
+    assert np.linalg.norm(y - d) < 1e-6 * np.linalg.norm(d)
+    A.close()
+    h.close()

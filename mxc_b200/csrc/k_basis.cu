@@ -721,8 +721,9 @@ __global__ void __launch_bounds__(128) k_pivchol_update(const i64* __restrict__ 
                                                         int k0) {
   constexpr int LD = PC_T + 4;
   const int box = blockIdx.x, M = (int)dims[box], steps = (int)steps_box[box];
+  if (M == 0 || k0 + PC_NB >= steps) return;  // no pivot left to take
   const int nt = (M + PC_T - 1) / PC_T, r0 = (int)blockIdx.y / nt * PC_T, c0 = (int)blockIdx.y % nt * PC_T;
-  if (M == 0 || k0 + PC_NB >= steps || r0 >= M) return;  // no pivot left to take
+  if (r0 >= M) return;
   __shared__ double As[PC_NB][LD], Bs[PC_NB][LD];
   const double* R = Rws + qoff[box] + (i64)k0 * M;
   double* g = G + qoff[box];

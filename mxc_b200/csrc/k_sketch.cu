@@ -53,6 +53,10 @@ __device__ __forceinline__ void sk_dmma(double (&d)[2], double a, double b) {
                : "d"(a), "d"(b));
 }
 
+// Barrier of the whole block that its warps reach at different places, each
+// warp as one (__syncthreads() would have to be the same one for all threads).
+__device__ __forceinline__ void sk_barrier() { asm volatile("bar.sync 0;" ::: "memory"); }
+
 // Body index of entry f (0 <= f < S) of a box's far list: ranges r0..r1-1
 // hold [rstart[r], rstart[r] + count) with rend[r] the running count; the
 // walk starts at a range known to begin at or before f.
@@ -174,13 +178,13 @@ __global__ void __launch_bounds__(64 * WM + 32, sketch_ctas(WM))
     body1 = body_of(s0 + 1);
     load(body1);
     body2 = body_of(s0 + 2);
-    __syncthreads();
+    sk_barrier();
     for (int sl = s0; sl < s1; sl++) {
       publish(sl + 1, body1);
       body1 = body2;
       load(body1);
       body2 = body_of(sl + 3);
-      __syncthreads();
+      sk_barrier();
     }
     return;
   }
@@ -191,7 +195,7 @@ __global__ void __launch_bounds__(64 * WM + 32, sketch_ctas(WM))
 #pragma unroll
     for (int j = 0; j < 4; j++) acc[i][j][0] = acc[i][j][1] = 0.;
 
-  __syncthreads();
+  sk_barrier();
   const int wm = warp >> 1, wn = warp & 1;
   const int row32 = a0 + 32 * wm;                      // the warp's first row
   const int wsel = (row32 >> 6) - (a0 >> 6);           // its sign word
@@ -206,7 +210,7 @@ __global__ void __launch_bounds__(64 * WM + 32, sketch_ctas(WM))
                              xs[3 * cl + 2]);
       xf[b][cl * SK_CS + fl] = v;
     }
-    __syncthreads();
+    sk_barrier();
     const double* bs = xf[b] + (wn * 32 + (lane >> 2)) * SK_CS + (lane & 3);
 #pragma unroll
     for (int ks = 0; ks < SK_KS; ks += 4) {

@@ -22,3 +22,13 @@ def test_cluster_barrier_before_first_and_after_last_remote_access():
             sync = [x.start() for x in re.finditer(r"\bcl\.sync\(\)", body)]
             assert sync and sync[0] < use[0] and sync[-1] > use[-1], path
     assert seen
+
+
+def test_warps_with_tasks_of_their_own_do_not_meet_at_syncthreads():
+    """__syncthreads() has to be the same statement for every thread of a
+    block: a kernel whose preparing warp returns from its own loop uses the
+    barrier instruction instead."""
+    text = re.sub(r"//[^\n]*", "", open(os.path.join(ROOT, "mxc_b200", "csrc", "k_sketch.cu")).read())
+    body = next(x for x in re.split(r"\b__global__\b", text)[1:] if "k_sketch(" in x)
+    body = body[:body.index("\n}")]
+    assert "__syncthreads" not in body and body.count("sk_barrier()") == 4

@@ -50,6 +50,32 @@ def test_bf16_apply_matches_fp32_apply(sys8k, nrhs):
         assert 1e-6 < e < 3e-2, (c, e)  # BF16-level agreement (and not FP32-level: the BF16 path ran)
 
 
+@pytest.mark.parametrize("n,nrhs", [(1, 1), (33, 1), (64, 2), (100, 3), (257, 4), (700, 2), (300, 8), (511, 16),
+                                    (700, 8), (650, 16)])
+def test_bf16_apply_of_one_box(handle, n, nrhs):
+    """A tree of one box: the substitution is the BF16 copy of the inverse
+    (exported in FP32) times the right-hand sides in FP32.  By rows, each
+    element is within the bound of a sum of n FP32 products; the tensor-core
+    kernel (the last two: sums over 512) also cuts B to two BF16 terms, 2^-17
+    of it."""
+    import torch
+
+    b = np.random.default_rng(n).random((n, 3))
+    handle.set_option(m._lib.OPT_PRECOND_BF16, 1)
+    try:
+        M = m.H2MatrixSolver(handle, m.Laplace3D(1e-2), 0.0, 8, 0, m.build_tree(b, 0), 2.0, b, precision=m.FP32)
+    finally:
+        handle.set_option(m._lib.OPT_PRECOND_BF16, 0)
+    M.factorizeM()
+    V = torch.from_numpy(M.export(0, m._lib.EXPORT_R).reshape(n, n).astype(np.float32)).bfloat16().double().numpy()
+    x = np.asfortranarray(np.random.default_rng(1).standard_normal((n, nrhs)).astype(np.float32).astype(float))
+    y = x.copy(order="F")
+    M.solvePrecondition(y if nrhs > 1 else y[:, 0])
+    eps = (n + 8) * 2.0 ** -24 + (2.0 ** -17 if n > 512 and nrhs > 4 else 0.0)
+    assert np.all(np.abs(y - V @ x) <= eps * (np.abs(V) @ np.abs(x)))
+    M.close()
+
+
 def test_bf16_preconditioned_gmres_reaches_dense_tolerance(sys8k, handle):
     A, M32, Mbf, k, b = sys8k
     N = b.shape[0]

@@ -96,10 +96,12 @@ def test_fp32_simt_gemm_same_bound(handle, case):
     assert worst < 1e-5, worst
 
 
-# Outputs of at most 16 columns with A and B as stored go to the streaming
-# kernels of the block-sparse applies (FP32: TF32 mma.sync with the split in
-# registers; FP64: mma.sync m8n8k4), rows in 128- and 256-row tiles; long
-# single entries are cut along k and their partials summed in order.
+# Outputs of at most 16 columns with A and B as stored go to the block-sparse
+# applies: by rows with at most 4 columns, or few row tiles and sums of at most
+# 512 (the first, third and fifth case); else to the streaming kernels (FP32:
+# TF32 mma.sync with the split in registers; FP64: mma.sync), rows in 128- and
+# 256-row tiles, long single entries cut along k and their partials summed in
+# order.
 SKINNY = [
     # batch, nterms, m, n, k, opA, opB, alpha, beta, lda, ldb, ldc
     (3, 1, 256, 16, 256, 0, 0, 1.0, 0.0, 256, 256, 256),
@@ -107,6 +109,15 @@ SKINNY = [
     (4, 2, 130, 8, 77, 0, 0, 0.5, 2.0, 131, 77, 130),
     (2, 1, 700, 16, 900, 0, 0, 1.0, 1.0, 700, 900, 701),
     (2, 1, 45, 3, 33, 0, 0, 1.0, 0.0, 45, 33, 45),
+]
+
+
+# Streaming kernels with 5 to 8 columns: sums over 512 with leading dimensions
+# that allow 16-byte (FP64: bulk) copies and not, more than 256 row tiles.
+SKINNY += [
+    (3, 2, 300, 8, 600, 0, 0, -1.0, 1.0, 300, 600, 300),
+    (2, 1, 130, 5, 700, 0, 0, 1.0, 0.0, 131, 701, 130),
+    (300, 1, 128, 7, 64, 0, 0, 1.0, 2.0, 128, 64, 128),
 ]
 
 

@@ -24,8 +24,9 @@ namespace h2b {
 // AP_KC NW columns, the sum over the warps -- about 8 us a launch at K 256,
 // where the shared-memory ring took 15 with the launch that adds its partial
 // sums.  With at most 4 columns also the faster kernel where HBM bounds it (4.5
-// TB/s against 3.7); with 16 the ring is (a warp reads 256 or 512 bytes of a
-// column here, the ring 512 to 2,048).
+// TB/s against 3.7; the exception is a substitution of 262,144 bodies in FP32
+// with one or two columns, 1,608 against 1,583 us); with 16 the ring is (a warp
+// reads 256 or 512 bytes of a column here, the ring 512 to 2,048).
 constexpr int AP_KC = 16, AP_EMAX = 64;
 
 template <typename AT, typename T>

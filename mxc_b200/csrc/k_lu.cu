@@ -427,7 +427,7 @@ cudaError_t launch_lu_solve(const LuSolveTask<T>* d_tasks, int ntasks, int maxn,
   if (maxn > 2048) return cudaErrorInvalidValue;  // rows of a panel held in registers
   const size_t ints = (3 * sizeof(int) * (size_t)maxn + 15) / 16 * 16;
   const size_t mat = sizeof(T) * (size_t)maxn * (maxn | 1);
-  // Static tiles take up to 51 KB (FP64, NB 32) of the 227 KB.
+  // The static tiles take up to 42 KB (FP64, NB 32) of the 227 KB.
   const bool in_smem = maxn <= 256 && ints + mat <= 168 * 1024;
   const size_t smem = ints + (in_smem ? mat : 0) + 16;
   auto go = [&](auto kern, int nt) {

@@ -85,11 +85,14 @@ __device__ __forceinline__ i64 sk_body(i64 f, i64 from, i64 r0, const i64* __res
 // chip's last wave badly (k_sketch_sum adds them).  20,000 bodies, five levels: 20.5 -> 14.4 ms (19.5 TFLOP/s of
 // the 36.8 of the pipe; leaves of 312 bodies 12.9 -> 9.2) against 128-row tiles
 // in one piece, the slab's far bodies fetched by a multiplying warp.
-// CTAs per SM by registers (about 100 a thread).
+// CTAs per SM.  They leave a thread 80 registers with 3 or 10 row groups, 96 with
+// 4, 8 or 9 and up to 128 otherwise; with the 64 of the accumulators that is
+// tight: Laplace spills 220 bytes at 80, 16 to 60 at 96 and none beyond (every
+// kind: 336, up to 76, none).
 __host__ __device__ constexpr int sketch_ctas(int wm) { return wm <= 3 ? 3 : wm <= 4 ? 2 : 1; }
 
 // KIND: the kernel kind where it is known at compile time (Laplace: without the
-// other kinds' sincos and exp no accumulator is spilled), -1 to read kp_in.
+// other kinds' sincos and exp a third less is spilled), -1 to read kp_in.
 template <int WM, int KIND>
 __global__ void __launch_bounds__(64 * WM + 32, sketch_ctas(WM))
     k_sketch(KernelParams kp_in, const double* __restrict__ bodies, const double* __restrict__ pts,

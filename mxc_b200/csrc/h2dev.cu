@@ -387,10 +387,14 @@ static int tuned_variant(const std::string& key, int nvar, cudaStream_t st, F ru
 
 // Whether a streaming plan runs by rows (k_apply): with at most 4 right-hand
 // sides always (near field of 20,000 bodies, 1 column: 186 -> 150 us; a level's
-// small pass 15 -> 8.5), with more only where the latency of a launch counts --
-// few row tiles and short sums (16 columns, K 256: 128 boxes 27 -> 25 us, 16
-// boxes 17 -> 12.5, but 512 boxes 52 -> 72; sums over 27 neighbours, K 3456:
-// 128 boxes 76 -> 109 us), where the ring's split tasks need a second launch.
+// small pass 15 -> 8.5), with more only where the latency of a launch counts,
+// since the ring's split tasks need a second launch -- few row tiles and short
+// sums.  Against the ring, 16 columns: 32 row tiles, sums of 256 13.5 and 21.8 us
+// in FP64, 11.5 and 19.8 in FP32; 256 tiles, sums of 512 36 and 40 in FP32, of 768
+// 59 and 48.  FP64 gains up to 128 tiles (sums of 256 21.9 and 21.3) and a plan of
+// 256 alone loses (77 and 54 at 512), but passes do not (a limit of 128: products
+// of 50,001 bodies, 8 columns, 1,119 -> 1,139 us; substitution of 32,768, 743 ->
+// 731), so one limit serves all.
 template <typename TK, typename EN>
 static bool apply_by_rows(int nr, const std::vector<TK>& tasks, const std::vector<EN>& ents) {
   if (nr <= 4) return true;

@@ -942,7 +942,7 @@ struct BfPlan {
   void run(cudaStream_t st) const {
     Prof p("bf16_precond", flops, bytes, st);
     if (by_rows) {
-      ck(launch_apply_bf16(nr, 2, d_tasks.p, d_ents.p, d_tiles.p, (int)tiles.size(), st), "apply_bf16");
+      ck(launch_apply_bf16(nr, d_tasks.p, d_ents.p, d_tiles.p, (int)tiles.size(), st), "apply_bf16");
       return;
     }
     ck(launch_stream_bf16(nr, d_tasks.p, d_ents.p, d_tiles.p, (int)tiles.size(), st), "bf16_precond");

@@ -53,7 +53,6 @@ template <> struct ApVec<float, 1> { using V = float; };
 template <> struct ApVec<float, 2> { using V = float2; };
 template <> struct ApVec<double, 1> { using V = double; };
 template <> struct ApVec<double, 2> { using V = double2; };
-template <> struct ApVec<__nv_bfloat16, 1> { using V = __nv_bfloat16; };
 template <> struct ApVec<__nv_bfloat16, 2> { using V = __nv_bfloat162; };
 
 __device__ __forceinline__ float ap_up(float v) { return v; }
@@ -236,7 +235,9 @@ static cudaError_t apply_any(int nr, int rl, const GemmTask<T>* tasks, const ENT
     if constexpr (sizeof(T) == 4 || N > 8) {                                                     \
       if (rl == 2) return apply_go<AT, T, ENT, N, 2, 8>(tasks, ents, tiles, ntiles, st);         \
     }                                                                                            \
-    if (rl == 1) return apply_go<AT, T, ENT, N, 1, 8>(tasks, ents, tiles, ntiles, st);           \
+    if constexpr (sizeof(AT) >= 4) {                                                             \
+      if (rl == 1) return apply_go<AT, T, ENT, N, 1, 8>(tasks, ents, tiles, ntiles, st);         \
+    }                                                                                            \
   }
   H2B_APPLY(1)
   H2B_APPLY(2)
@@ -256,9 +257,9 @@ template cudaError_t launch_apply<double>(int, int, const GemmTask<double>*, con
                                           int, cudaStream_t);
 template cudaError_t launch_apply<float>(int, int, const GemmTask<float>*, const GemmEntry<float>*, const int2*, int,
                                          cudaStream_t);
-cudaError_t launch_apply_bf16(int nr, int rl, const GemmTask<float>* tasks, const BfEntry* ents, const int2* tiles,
-                              int ntiles, cudaStream_t st) {
-  return apply_any<__nv_bfloat16, float, BfEntry>(nr, rl, tasks, ents, tiles, ntiles, st);
+cudaError_t launch_apply_bf16(int nr, const GemmTask<float>* tasks, const BfEntry* ents, const int2* tiles, int ntiles,
+                              cudaStream_t st) {
+  return apply_any<__nv_bfloat16, float, BfEntry>(nr, 2, tasks, ents, tiles, ntiles, st);
 }
 
 }  // namespace h2b

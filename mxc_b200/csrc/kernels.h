@@ -230,13 +230,15 @@ struct BfEntry {
   float alpha;
   const float* scale;
 };
-cudaError_t launch_apply_bf16(int nr, int rl, const GemmTask<float>* d_tasks, const BfEntry* d_ents,
-                              const int2* d_tiles, int ntiles, cudaStream_t st);
 cudaError_t launch_bf16_pack(const BfPackTask* d_tasks, int ntasks, cudaStream_t st);
 // 5-16 right-hand sides on the BF16 tensor cores (k_stream_bf16_mma).
 cudaError_t launch_stream_bf16(int nr, const GemmTask<float>* d_tasks, const BfEntry* d_ents, const int2* d_tiles,
                                int ntiles, cudaStream_t st);
 int bf16_rows_per_cta();
+// The same products by rows (k_apply.cu), up to 16 right-hand sides, tiles of
+// apply_rows_per_cta(2) rows.
+cudaError_t launch_apply_bf16(int nr, const GemmTask<float>* d_tasks, const BfEntry* d_ents, const int2* d_tiles,
+                              int ntiles, cudaStream_t st);
 
 template <typename T>
 struct CopyEntry {
